@@ -267,7 +267,8 @@ typedef struct
   int32_t state;           /* 0: not tuned yet, 1: measured, 2: from the process cache, 3: fixed */
   int32_t update_variant;  /* 0/1/6: one thread per neuron (4/8/2 lags of inputs at a time), 2/3:
                               two-phase (256/128-thread CTAs), 4: aeif_cond_alpha's RKF45 kernel,
-                              5: the persistent slice kernel */
+                              5: the persistent slice kernels (the target-owning one where the
+                              network suits it) */
   int32_t deliver_per_sm;  /* resident delivery CTAs per SM */
   int32_t deliver_group;   /* edge chunks per delivery warp and descriptor load */
   int32_t cache_hit;

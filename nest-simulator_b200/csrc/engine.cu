@@ -27,6 +27,7 @@
 #include "../../include/nestgpu.h"
 #include "ng_kernels.cuh"
 #include "ng_persistent.cuh"
+#include "ng_owned.cuh"
 #include "ng_serving.cuh"
 #include "ng_stdp.cuh"
 
@@ -725,6 +726,16 @@ struct ng_engine
                              // kernel (update and delivery of many slices in one launch); -1: by
                              // network size (serving engines: 6)
   DevBuf pk;                 // grid-barrier state of the persistent slice kernel
+  // ---- target-owning slice kernel (k_run_owned): the owners' copy of the
+  // in-edges, laid out for the network as it is connected now
+  int own_state = 0;         // 0: to be built, 1: ready, -1: the network does not qualify
+  bool own_drive_ok = true;  // every drive table is a CDF table (no walk from the mode)
+  DevBuf own_cta, own_rpb, own_rp, own_eb, own_rpf, own_ebf, own_word, own_weight, own_x;
+  bool own_held = true;
+  int own_cell = 0, own_grid = 0, own_net = -1;
+  size_t own_smem_bytes = 0;
+  OwnNet own_net_d {};
+  uint64_t own_seq = 0;      // slices published so far (tags of the exchange buffer)
   // ---- stdp_pl_synapse_hom connections (ng_set_plastic_connections)
   bool plastic_on = false;
   DevBuf pl_row, pl_tgt, pl_dly, pl_w, pl_Kplus, pl_tlast, pl_ninc, pl_tauinv, pl_Kminus, pl_last, pl_hist_t, pl_hist_K,
@@ -797,7 +808,7 @@ struct ng_engine
       &net_spk, &log_sorted, &log_cnt, &log_off, &sc_bound, &seg, &net_t, &row_ue, &row_ls, &ent_late, &pk, &pl_row,
       &pl_tgt, &pl_dly, &pl_w, &pl_Kplus, &pl_tlast, &pl_ninc, &pl_tauinv, &pl_Kminus, &pl_last, &pl_hist_t, &pl_hist_K,
       &pl_hist_n, &pl_hist_lo, &pl_drop_t, &pl_drop_K, &pl_nflush, &pl_in_row, &pl_in_edge, &pl_in_src, &pl_wrun,
-      &pl_tab_fin, &pl_tab_km };
+      &pl_tab_fin, &pl_tab_km, &own_cta, &own_rpb, &own_rp, &own_eb, &own_rpf, &own_ebf, &own_word, &own_weight, &own_x };
     for ( DevBuf* b : bufs )
       cudaFree( b->p );
     if ( host_ctl )
@@ -1233,6 +1244,406 @@ struct ng_engine
     return N > ( int64_t ) pk_occ * sms * PK_NB;
   }
 
+  // ---- target-owning slice kernel
+  template < typename Real, bool FIX, int MODEL, int CELL >
+  const void*
+  own_func( bool held ) const
+  {
+    return held ? reinterpret_cast< const void* >( &k_run_owned< Real, FIX, MODEL, CELL, true > )
+                : reinterpret_cast< const void* >( &k_run_owned< Real, FIX, MODEL, CELL, false > );
+  }
+
+  template < int MODEL >
+  const void*
+  own_func_m( int cell, bool held ) const
+  {
+    if ( prec == NG_FP64 )
+      return cell == OW_COUNT ? own_func< double, false, MODEL, OW_COUNT >( held )
+                              : own_func< double, false, MODEL, OW_F64 >( held );
+    return cell == OW_COUNT ? own_func< float, true, MODEL, OW_COUNT >( held )
+                            : own_func< float, true, MODEL, OW_I64 >( held );
+  }
+
+  const void*
+  own_kernel( int cell, bool held ) const
+  {
+    const int m = blk[ 0 ].model;
+    return m == NG_IAF_PSC_DELTA ? own_func_m< NG_IAF_PSC_DELTA >( cell, held )
+      : m == NG_IAF_PSC_EXP      ? own_func_m< NG_IAF_PSC_EXP >( cell, held )
+                                 : own_func_m< NG_IAF_PSC_ALPHA >( cell, held );
+  }
+
+  // the network that k_run_owned can take: the neurons of a static engine
+  // (or the one live network of a serving engine without gather tables) of
+  // one iaf model, without scheduled or plastic spikes
+  bool
+  own_possible( int64_t* a, int64_t* n, int* net_id ) const
+  {
+    if ( blk.size() != 1 || blk[ 0 ].model == NG_AEIF_COND_ALPHA || n_sched > 0 || plastic_on || tiled_on
+      || ring_bytes != 8 || !own_drive_ok || cfg.min_delay >= ( 1 << ( 32 - OW_SBITS ) )
+      || cfg.max_delay >= ( 1 << 20 ) )
+      return false;
+    *a = 0;
+    *n = N;
+    *net_id = -1;
+    if ( serving )
+    {
+      for ( size_t id = 0; id < nets.size(); ++id )
+        if ( nets[ id ].used )
+        {
+          if ( *net_id >= 0 )
+            return false;
+          *net_id = ( int ) id;
+          *a = nets[ id ].off;
+          *n = nets[ id ].n;
+        }
+      if ( *net_id < 0 || nets[ ( size_t ) *net_id ].ne <= 0
+        || ( gather_on && host_g[ ( size_t ) *net_id ].ke + host_g[ ( size_t ) *net_id ].ki > 0 ) )
+        return false;
+    }
+    else if ( nnz_padded <= 0 )
+      return false;
+    return *n <= ( int64_t ) sms * 2 * OW_TPB && *n < ( 1 << OW_SBITS ) && sms <= OW_MAX_G;
+  }
+
+  // the owners' layout: built at the first call after the graph changed.  A
+  // network it does not suit (or that does not fit) keeps the other kernels.
+  bool
+  own_ready()
+  {
+    int64_t a = 0, n = 0;
+    int id = -1;
+    if ( !own_possible( &a, &n, &id ) )
+      return false;
+    if ( own_state == 0 )
+    {
+      own_state = own_build( a, n, id ) == NG_OK ? 1 : -1;
+      if ( own_state < 0 )
+        cudaGetLastError();
+    }
+    return own_state > 0;
+  }
+
+  // Contiguous, mutually unconnected parts of the network (the copies of a
+  // batch): each gets SMs of its own, so a spike is exchanged and looked up
+  // among its own part's only.  More parts than SMs: one part.
+  int
+  own_parts( int64_t a, int64_t n, std::vector< OwnCta >& cta, int* nl )
+  {
+    std::vector< std::pair< int, int > > part;  // [first, end) of each part
+    std::vector< int64_t > load;
+    if ( !serving )
+    {
+      void* d_span = nullptr;
+      CU( cudaMalloc( &d_span, ( size_t ) n * sizeof( int2 ) ) );
+      std::vector< int2 > span( ( size_t ) n );
+      std::vector< int32_t > deg( ( size_t ) n );
+      k_own_span<<< ( unsigned ) ( ( n * 32 + 255 ) / 256 ), 256, 0, stream >>>( n, ( const int64_t* ) row_beg.p,
+        ( const int32_t* ) real_deg.p, ( const uint32_t* ) tdc.p, tmask, ( int2* ) d_span );
+      cudaError_t ce = cudaGetLastError();
+      if ( ce == cudaSuccess )
+        ce = cudaMemcpyAsync( span.data(), d_span, ( size_t ) n * sizeof( int2 ), cudaMemcpyDeviceToHost, stream );
+      if ( ce == cudaSuccess )
+        ce = cudaMemcpyAsync( deg.data(), real_deg.p, ( size_t ) n * 4, cudaMemcpyDeviceToHost, stream );
+      if ( ce == cudaSuccess )
+        ce = cudaStreamSynchronize( stream );
+      cudaFree( d_span );
+      CU( ce );
+      for ( int64_t s = 0; s < n; ++s )
+      {
+        int lo = std::min( ( int ) s, span[ ( size_t ) s ].x ), hi = std::max( ( int ) s, span[ ( size_t ) s ].y ) + 1;
+        int64_t e = deg[ ( size_t ) s ] + 1;
+        while ( !part.empty() && part.back().second > lo )
+        {
+          lo = std::min( lo, part.back().first );
+          hi = std::max( hi, part.back().second );
+          e += load.back();
+          part.pop_back();
+          load.pop_back();
+        }
+        part.emplace_back( lo, hi );
+        load.push_back( e );
+      }
+    }
+    if ( part.empty() || ( int64_t ) part.size() > sms )
+    {
+      part.assign( 1, { ( int ) a, ( int ) ( a + n ) } );
+      load.assign( 1, 1 );
+    }
+    // SMs per part: one each, then one at a time to the part with the most
+    // edges per SM, down to OWN_MIN_NEURONS neurons per SM
+    const size_t K = part.size();
+    std::vector< int > G( K, 1 );
+    for ( int left = sms - ( int ) K; left > 0; --left )
+    {
+      size_t best = K;
+      for ( size_t k = 0; k < K; ++k )
+        if ( ( int64_t ) G[ k ] * OWN_MIN_NEURONS < part[ k ].second - part[ k ].first
+          && ( best == K || load[ k ] * G[ best ] > load[ best ] * G[ k ] ) )
+          best = k;
+      if ( best == K )
+        break;
+      ++G[ best ];
+    }
+    cta.clear();
+    *nl = 0;
+    for ( size_t k = 0; k < K; ++k )
+    {
+      const int pn = part[ k ].second - part[ k ].first, c0 = ( int ) cta.size();
+      *nl = std::max( *nl, ( pn + G[ k ] - 1 ) / G[ k ] );
+      for ( int g = 0; g < G[ k ]; ++g )
+        cta.push_back( OwnCta { part[ k ].first, pn, c0, G[ k ] } );
+    }
+    return NG_OK;
+  }
+  // fewest neurons per SM: below it a network's spikes come from more SMs than
+  // they have work for (each polls every other one's)
+  static constexpr int OWN_MIN_NEURONS = 16;
+
+  template < typename T >
+  int
+  own_build_t( int64_t a, int64_t n, int id )
+  {
+    std::vector< OwnCta > cta;
+    int n_loc = 0, rc;
+    if ( ( rc = own_parts( a, n, cta, &n_loc ) ) )
+      return rc;
+    if ( n_loc > 2 * OW_TPB )
+      return NG_ERR_CAPACITY;
+    const int grid = ( int ) cta.size(), nl = n_loc + 1;  // (one column more for the segments' padding)
+    const bool fx = prec != NG_FP64, two = blk[ 0 ].model != NG_IAF_PSC_DELTA;
+    std::vector< long long > rpb( ( size_t ) grid );
+    long long rp_n = 0;
+    int n_max = 0;
+    for ( int c = 0; c < grid; ++c )
+    {
+      rpb[ ( size_t ) c ] = rp_n;
+      rp_n += cta[ ( size_t ) c ].n + 1;
+      n_max = std::max( n_max, cta[ ( size_t ) c ].n );
+    }
+    if ( ( rc = upload( own_cta, cta.data(), cta.size() * sizeof( OwnCta ) ) )
+      || ( rc = upload( own_rpb, rpb.data(), rpb.size() * 8 ) ) || ( rc = alloc( own_rp, ( size_t ) rp_n * 4 ) ) )
+      return rc;
+    // scratch: class weight bounds, owners' edge totals, in-degrees per class
+    struct Tmp
+    {
+      void* p = nullptr;
+      ~Tmp() { cudaFree( p ); }
+    } tmp;
+    const size_t head = 64 + ( size_t ) grid * 8;
+    CU( cudaMalloc( &tmp.p, head + ( size_t ) n * 8 ) );
+    unsigned long long* const bounds = ( unsigned long long* ) tmp.p;  // min[2], max[2], in-degree maximum
+    unsigned long long* const total = bounds + 8;
+    unsigned* const indeg = ( unsigned* ) ( ( char* ) tmp.p + head );
+    CU( cudaMemsetAsync( tmp.p, 0, head + ( size_t ) n * 8, stream ) );
+    CU( cudaMemsetAsync( bounds, 0xff, 16, stream ) );
+    OwnBuild q {};
+    q.row_beg = ( const int64_t* ) row_beg.p;
+    q.real_deg = ( const int32_t* ) real_deg.p;
+    q.tdc = ( const uint32_t* ) tdc.p;
+    q.w = w.p;
+    q.tmask = tmask;
+    q.dmask = dmask;
+    q.tbits = tbits;
+    q.rp_base = ( const long long* ) own_rpb.p;
+    auto each_part = [ & ]( auto&& f ) {
+      for ( int c = 0; c < grid; c += cta[ ( size_t ) c ].G )
+      {
+        q.a = cta[ ( size_t ) c ].a;
+        q.n = cta[ ( size_t ) c ].n;
+        q.c0 = c;
+        q.G = cta[ ( size_t ) c ].G;
+        f( ( unsigned ) std::min( ( q.n + 7 ) / 8, 8 * sms ) );
+      }
+    };
+    std::vector< unsigned long long > host( 8 + ( size_t ) grid );
+    // edges of delay [lo, hi) per owner and source as segment starts; owners' starts and total [quads]
+    auto count = [ & ]( DevBuf& rp, int lo, int hi, bool stats, std::vector< long long >& eb, long long* quads ) -> int {
+      q.rp = ( uint32_t* ) rp.p;
+      q.d_lo = lo;
+      q.d_hi = hi;
+      each_part( [ & ]( unsigned g ) {
+        k_own_count< T ><<< g, 256, 0, stream >>>( q, two ? 0 : 1, stats ? indeg - 2 * a : nullptr, bounds, bounds + 2 );
+      } );
+      if ( stats )
+        k_own_max<<< ( unsigned ) std::min< int64_t >( ( 2 * n + 255 ) / 256, 4 * sms ), 256, 0, stream >>>( 2 * n, indeg,
+          ( unsigned* ) ( bounds + 4 ) );
+      k_own_scan<<< ( unsigned ) grid, 1024, 0, stream >>>( ( const OwnCta* ) own_cta.p, ( const long long* ) own_rpb.p,
+        ( uint32_t* ) rp.p, total );
+      CU( cudaGetLastError() );
+      CU( cudaMemcpyAsync( host.data(), tmp.p, head, cudaMemcpyDeviceToHost, stream ) );
+      CU( cudaStreamSynchronize( stream ) );
+      eb.assign( ( size_t ) grid, 0 );
+      *quads = 0;
+      for ( int c = 0; c < grid; ++c )
+      {
+        eb[ ( size_t ) c ] = *quads;
+        *quads += ( long long ) host[ 8 + ( size_t ) c ];
+      }
+      return NG_OK;
+    };
+    std::vector< long long > eb, ebf;
+    long long quads = 0, quads_far = 0;
+    if ( ( rc = count( own_rp, 0, INT32_MAX, true, eb, &quads ) ) )
+      return rc;
+    // (a cell's 16-bit event count and 16 high bits hold any in-degree up to this)
+    if ( quads == 0 || ( unsigned ) host[ 4 ] > 65000u )
+      return NG_ERR_CAPACITY;
+    // one weight per input class: cells count events
+    OwnNet o {};
+    bool uniform = true;
+    for ( int c = 0; c < 2; ++c )
+    {
+      const unsigned long long mn = host[ ( size_t ) c ], mx = host[ 2 + ( size_t ) c ];
+      if ( mx == 0 )
+        continue;  // no edge of this class
+      uniform = uniform && mn == mx;
+      if ( fx )
+        o.cwi[ c ] = ( int ) ( ( long long ) mx - ( 1ll << 40 ) );
+      else
+      {
+        const unsigned long long u = ( mx >> 63 ) ? mx & ~( 1ull << 63 ) : ~mx;
+        std::memcpy( &o.cw[ c ], &u, 8 );
+      }
+    }
+    const int cell = uniform ? OW_COUNT : fx ? OW_I64 : OW_F64;
+    // ring window: all delays where they fit, else the nearest ones, beside the
+    // stage of at least 4 lags' inputs (all of the slice's where there is room)
+    int optin = 0;
+    CU( cudaDeviceGetAttribute( &optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg.device ) );
+    const size_t room = ( size_t ) optin - 4096;  // (static shared memory)
+    const int md = cfg.min_delay, rsz_i = ( int ) rsz;
+    const bool held = n_loc <= OW_TPB;
+    int kc = std::min( md, 4 );
+    const size_t fixed = own_smem( cell, two, held, nl, 0, md, rsz_i, kc, 0 ).total;
+    if ( fixed >= room )
+      return NG_ERR_CAPACITY;
+    const int W = ( int ) std::min< size_t >( ( size_t ) L, ( room - fixed ) / ( ( size_t ) nl * own_cell_bytes( cell, two ) ) );
+    // a window below min_delay + 16 slots would send most arrivals through the
+    // global ring, the scatter form's path
+    if ( W < L && W < md + 16 )
+      return NG_ERR_CAPACITY;
+    while ( kc < std::min( md, 32 ) && own_smem( cell, two, held, nl, W, md, rsz_i, kc + 1, 0 ).total <= room )
+      ++kc;
+    o.kc = kc;
+    o.rp_smem = own_smem( cell, two, held, nl, W, md, rsz_i, kc, n_max + 1 ).total <= room ? 1 : 0;
+    own_smem_bytes = own_smem( cell, two, held, nl, W, md, rsz_i, kc, o.rp_smem ? n_max + 1 : 0 ).total;
+    own_held = held;
+    own_cell = cell;
+    own_grid = grid;
+    own_net = id;
+    o.far = W < L ? 1 : 0;
+    if ( o.far )
+    {
+      // an edge of delay d arrives d - 1 steps past the next slice's first one at most
+      if ( ( rc = alloc( own_rpf, ( size_t ) rp_n * 4 ) ) || ( rc = count( own_rp, 0, W + 1, false, eb, &quads ) )
+        || ( rc = count( own_rpf, W + 1, INT32_MAX, false, ebf, &quads_far ) ) )
+        return rc;
+    }
+    o.x_cap = std::max< long long >( 32, ( long long ) nl * md + 1 );
+    // 2-byte edge words where (delay, local target) fits 15 bits
+    o.w16 = cell == OW_COUNT && ( int64_t ) ( cfg.max_delay + 1 ) * nl < 32768 ? 1 : 0;
+    const size_t wb = cell == OW_I64 ? 8 : o.w16 ? 2 : 4;
+    if ( ( rc = alloc( own_x, 2 * ( size_t ) grid * ( size_t ) o.x_cap * 8 ) )
+      || ( !pk.p && ( rc = alloc( pk, sizeof( PkCtl ) ) ) ) )
+      return rc;
+    own_seq = 0;
+    // near edges, then far ones, in one array each of words and weights
+    const size_t edges = 4 * ( size_t ) ( quads + quads_far );
+    for ( long long& x : ebf )
+      x += quads;
+    if ( ( rc = upload( own_eb, eb.data(), eb.size() * 8 ) ) || ( rc = upload( own_ebf, ebf.data(), ebf.size() * 8 ) )
+      || ( rc = alloc( own_word, edges * wb ) ) || ( rc = alloc( own_weight, cell == OW_F64 ? edges * 8 : 16 ) ) )
+      return rc;
+    k_own_pad<<< ( unsigned ) ( 16 * sms ), 256, 0, stream >>>( o.w16, cell == OW_I64 ? 1 : 0, edges,
+      ( uint32_t ) ( md * nl + nl - 1 ), ( uint32_t* ) own_word.p );
+    for ( int f = 0; f <= o.far; ++f )
+    {
+      q.rp = ( uint32_t* ) ( f ? own_rpf.p : own_rp.p );
+      q.d_lo = f ? W + 1 : 0;
+      q.d_hi = o.far && !f ? W + 1 : INT32_MAX;
+      each_part( [ & ]( unsigned g ) {
+        k_own_fill< T ><<< g, 256, 0, stream >>>( q, two ? 0 : 1, cell, o.w16, nl,
+          ( const long long* ) ( f ? own_ebf.p : own_eb.p ), ( uint32_t* ) own_word.p, ( uint2* ) own_word.p,
+          ( double* ) own_weight.p );
+      } );
+    }
+    CU( cudaGetLastError() );
+    CU( cudaFuncSetAttribute( own_kernel( cell, own_held ), cudaFuncAttributeMaxDynamicSharedMemorySize,
+      ( int ) own_smem_bytes ) );
+    int occ = 0, coop = 0;
+    CU( cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, cfg.device ) );
+    CU( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, own_kernel( cell, own_held ), OW_TPB, own_smem_bytes ) );
+    if ( !coop || occ < 1 )
+      return NG_ERR_CAPACITY;
+    CU( cudaStreamSynchronize( stream ) );
+    // lanes per segment, a quad of edges (OW_COUNT: two) each: 1.4 times the mean segment
+    double segs = 0;
+    for ( const OwnCta& c : cta )
+      segs += c.n;
+    const double mean = ( double ) quads / segs;
+    o.gw_log2 = 0;
+    while ( o.gw_log2 < 5 && ( double ) ( ( cell == OW_COUNT ? 2 : 1 ) << o.gw_log2 ) < 1.4 * mean )
+      ++o.gw_log2;
+    o.cta = ( const OwnCta* ) own_cta.p;
+    o.rp_base = ( const long long* ) own_rpb.p;
+    o.rp = ( const uint32_t* ) own_rp.p;
+    o.e_base = ( const long long* ) own_eb.p;
+    o.rp_far = ( const uint32_t* ) own_rpf.p;
+    o.e_far = ( const long long* ) own_ebf.p;
+    o.word = ( const uint4* ) own_word.p;
+    o.word_w = ( const uint4* ) own_word.p;
+    o.weight = ( const double2* ) own_weight.p;
+    o.xchg = ( unsigned long long* ) own_x.p;
+    o.nl = nl;
+    o.W = W;
+    o.pk = ( PkCtl* ) pk.p;
+    own_net_d = o;
+    return NG_OK;
+  }
+
+  int
+  own_build( int64_t a, int64_t n, int id )
+  {
+    return prec == NG_FP64 ? own_build_t< double >( a, n, id ) : own_build_t< int32_t >( a, n, id );
+  }
+
+  // full slices the target-owning kernel may run from here on (0: none): a
+  // serving engine's network must live through all of them
+  int64_t
+  own_slices( int64_t full )
+  {
+    if ( full < 1 || !own_ready() )
+      return 0;
+    if ( own_net >= 0 )
+      full = std::min< int64_t >( full, ( nets[ ( size_t ) own_net ].until - origin ) / cfg.min_delay );
+    return std::max< int64_t >( full, 0 );
+  }
+
+  int
+  launch_owned( const Net& d, int k )
+  {
+    Net dd = d;
+    Block db = dblock( blk[ 0 ] );
+    // tags are 32 bits wide: start over, with a cleared exchange buffer, long before they repeat
+    if ( own_seq + ( uint64_t ) k + 2 > 0xffffffffull )
+    {
+      CU( cudaMemsetAsync( own_x.p, 0, own_x.bytes, stream ) );
+      own_seq = 0;
+    }
+    own_net_d.seq0 = ( unsigned ) ( own_seq + 1 );
+    own_seq += ( uint64_t ) k;
+    own_net_d.origin0 = origin;
+    const size_t n_cdf = serving ? cdf_host.size() : pois_cdf.bytes / 8;
+    own_net_d.n_cdf = has_pois && n_cdf <= ( size_t ) OW_CDF ? ( int ) n_cdf : 0;
+    CU( cudaMemsetAsync( pk.p, 0, sizeof( PkCtl ), stream ) );
+    OwnNet o = own_net_d;
+    void* args[] = { &dd, &db, &o, &k };
+    CU( cudaLaunchCooperativeKernel( own_kernel( own_cell, own_held ), dim3( ( unsigned ) own_grid ),
+      dim3( ( unsigned ) OW_TPB ), args, own_smem_bytes, stream ) );
+    return NG_OK;
+  }
+
   // the persistent slice kernel applies: one iaf block of a static engine,
   // no traces or scheduled generator spikes (whose bookkeeping is per
   // launch), a device that supports cooperative launches
@@ -1548,13 +1959,18 @@ struct ng_engine
     const Net d = net();
     while ( n > 0 )
     {
-      if ( from == 0 && upd_variant == 5 && n >= cfg.min_delay && persistent_ok() )
+      // the persistent forms: the target-owning kernel where the network
+      // suits it -- also before tuning, from two slices on -- else the
+      // scatter form
+      const int64_t full = from == 0 ? n / cfg.min_delay : 0;
+      const int64_t owned = upd_variant == 5 || ( upd_variant < 0 && full > 1 ) ? own_slices( full ) : 0;
+      if ( full > 0 && ( owned > 0 || ( upd_variant == 5 && persistent_ok() ) ) )
       {
-        const int k = ( int ) std::min< int64_t >( n / cfg.min_delay, 1 << 20 );
+        const int k = ( int ) std::min< int64_t >( owned > 0 ? owned : full, 1 << 20 );
         late_join();
         if ( profiling )
           CU( cudaEventRecord( ev0, stream ) );
-        int rc = launch_persistent( d, k );
+        int rc = owned > 0 ? launch_owned( d, k ) : launch_persistent( d, k );
         if ( rc )
           return rc;
         if ( profiling )
@@ -2063,7 +2479,7 @@ struct ng_engine
         variants.push_back( 2 );
         variants.push_back( 3 );
       }
-      if ( persistent_ok() )
+      if ( own_ready() || persistent_ok() )
         variants.push_back( 5 );
     }
     std::vector< int > per_sm;
@@ -2787,6 +3203,7 @@ ng_set_connections( ng_engine* e, int64_t n_src, const int64_t* row_ptr, const i
   free_tmp();
   e->fx_inv = fx ? std::ldexp( 1.0, -S ) : 1.0;
   e->nnz_padded = np;
+  e->own_state = 0;
   e->chunks_all_src = 0;
   e->chunks_max_gen = 0;
   for ( int64_t sidx = 0; sidx < n_src; ++sidx )
@@ -3012,7 +3429,7 @@ ng_set_poisson( ng_engine* e, const double* rate_hz, const double* weight, const
   std::vector< int2 > ref( ( size_t ) n, make_int2( 0, 0 ) );
   std::vector< uint64_t > cdf;
   std::unordered_map< double, int2 > tables;  // one CDF table per distinct lambda
-  bool any = false;
+  bool any = false, tables_only = true;
   for ( int64_t i = 0; i < n; ++i )
   {
     if ( rate_hz[ i ] > 0 && ( delay_steps[ i ] < e->cfg.min_delay || delay_steps[ i ] > e->cfg.max_delay ) )
@@ -3036,7 +3453,9 @@ ng_set_poisson( ng_engine* e, const double* rate_hz, const double* weight, const
       it = tables.emplace( lam, r2 ).first;
     }
     ref[ i ] = it->second;
+    tables_only = tables_only && it->second.y > 0;
   }
+  e->own_drive_ok = tables_only;
   if ( cdf.empty() )
     cdf.push_back( 1ull << 53 );
   int rc;
@@ -3963,6 +4382,8 @@ ng_net_add( ng_engine* e, const ng_net_desc* desc, int32_t* net_id )
         it = e->cdf_tables.emplace( lam, r2 ).first;
       }
       ref[ i ] = it->second;
+      if ( it->second.y < 0 )
+        e->own_drive_ok = false;  // (for the engine's lifetime: networks with longer tables are rare)
     }
     const int64_t cdf_new = ( int64_t ) e->cdf_host.size();
     if ( cdf_new > cdf_old )
@@ -4013,6 +4434,7 @@ ng_net_add( ng_engine* e, const ng_net_desc* desc, int32_t* net_id )
   nw.sn = sgn;
   nw.step0 = step0;
   nw.until = until;
+  e->own_state = 0;
   nw.rec = desc->record != 0;
   nw.log_rate = desc->record ? log_rate : 0.0;
   e->n_rec += desc->record ? n : 0;
@@ -4250,6 +4672,7 @@ ng_net_remove( ng_engine* e, int32_t id )
   }
   e->n_rec -= nw.rec ? nw.n : 0;
   e->log_per_step = std::max( 1.0, e->log_per_step - nw.log_rate );
+  e->own_state = 0;
   ng_engine::free_blocks( nw.blocks );
   nw = ng_engine::NetInfo();
   e->refresh_late();
