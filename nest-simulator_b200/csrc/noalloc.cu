@@ -159,6 +159,245 @@ k_na_deliver( NaNet d )
   }
 }
 
+// ---------------------------------------------------------------------
+// A call on a network of up to NA_CL_CTAS x 1024 neurons in one launch: one
+// cluster of CTAs, one thread per neuron.  A CTA keeps its neurons' state in
+// registers and its own spikes of the open slice in shared memory, delivers
+// them itself when the slice closes (the ring holds min_delay + max_delay
+// slots, so a delivery meets no cell that another CTA still has to read), and
+// one cluster barrier per slice orders the deliveries before the next update.
+// The launches of the kernels above, three per slice, each with its fixed
+// cost, were the time of a controller's call: 213 us for ten slices of 1,000
+// neurons, 75 us in one launch.  The ring cells of up to NA_LAGS lags are
+// read ahead of the recurrence, whose lags would else wait for one L2 round
+// trip each.
+// ---------------------------------------------------------------------
+constexpr int NA_CL_CTAS = 8;   // (the portable cluster size)
+constexpr int NA_LAGS = 8;
+constexpr int NA_LIST = 1024 * NA_LAGS;  // a CTA's spikes held at a time
+
+__device__ __forceinline__ void
+na_cluster_sync()
+{
+  asm volatile( "barrier.cluster.arrive.release.aligned;" ::: "memory" );
+  asm volatile( "barrier.cluster.wait.acquire.aligned;" ::: "memory" );
+}
+
+// one warp: the edges of a spike (source, emission slot)
+__device__ __forceinline__ void
+na_deliver_spike( const NaNet& d, int src, int slot0, unsigned long long& skipped )
+{
+  const int64_t e1 = d.row_ptr[ src + 1 ];
+  for ( int64_t e0 = d.row_ptr[ src ] + ( threadIdx.x & 31 ); e0 < e1; e0 += 128 )
+  {
+    // four edges per lane in flight
+    int32_t tg[ 4 ], dl[ 4 ];
+    double w[ 4 ];
+#pragma unroll
+    for ( int u = 0; u < 4; ++u )
+    {
+      const int64_t e = e0 + 32 * u;
+      tg[ u ] = e < e1 ? d.target[ e ] : 0;
+      dl[ u ] = e < e1 ? d.delay[ e ] : 0;
+      w[ u ] = e < e1 ? d.weight[ e ] : 0.0;
+    }
+#pragma unroll
+    for ( int u = 0; u < 4; ++u )
+    {
+      if ( e0 + 32 * u >= e1 )
+        continue;
+      if ( tg[ u ] < 0 || ( int64_t ) tg[ u ] >= d.n || dl[ u ] < d.min_delay || dl[ u ] > d.max_delay )
+      {
+        ++skipped;
+        continue;
+      }
+      int slot = slot0 + dl[ u ];  // slot0 < L and dl <= max_delay < L
+      if ( slot >= d.L )
+        slot -= d.L;
+      atomicAdd( d.ring + ( int64_t ) slot * d.n + tg[ u ], w[ u ] );
+    }
+  }
+}
+
+__global__ void __launch_bounds__( 1024 )
+k_na_run( NaNet d, int per, long long start, long long n_steps, int fresh )
+{
+  __shared__ uint32_t s_list[ NA_LIST ];  // local neuron, lag of the chunk << 16
+  __shared__ int s_n;
+  __shared__ unsigned long long s_out;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int64_t i0 = ( int64_t ) blockIdx.x * per, i = i0 + tid;  // `per` neurons per CTA
+  const bool act = tid < per && i < d.n;
+  const bool first = blockIdx.x == 0 && tid == 0;
+  if ( fresh )
+  {
+    // counters and ring of a new run
+    for ( int64_t k = ( int64_t ) blockIdx.x * blockDim.x + tid; k < ( int64_t ) d.L * d.n;
+          k += ( int64_t ) gridDim.x * blockDim.x )
+      d.ring[ k ] = 0.0;
+    if ( first )
+      d.ctl->n_spk = 0ull;
+  }
+  if ( first )
+    d.ctl->n_out = d.ctl->n_skip = 0ull;
+  if ( tid == 0 )
+    s_n = 0;
+  double V = 0, P33 = 0, Vth = 0, Vreset = 0, Vmin = 0, drive = 0;
+  int r = 0, refr = 0;
+  if ( act )
+  {
+    const double y0 = 0.0;
+    V = d.V[ i ];
+    r = d.r[ i ];
+    P33 = d.P33[ i ];
+    Vth = d.V_th[ i ];
+    Vreset = d.V_reset[ i ];
+    Vmin = d.V_min[ i ];
+    refr = d.refr_counts[ i ];
+    drive = d.P30[ i ] * ( y0 + d.I_e[ i ] );
+  }
+  unsigned long long skipped = 0;
+  long long t = start;
+  const long long end = start + n_steps;
+  // spikes of the open slice that earlier calls left; where it closes in this
+  // call the list is emptied once every CTA has read its length (a slice left
+  // open at the end adds to it behind the first close's barrier)
+  const unsigned long long n_old = fresh ? 0ull : __ldcg( &d.ctl->n_spk );
+  const int64_t old = ( int64_t ) n_old < d.spk_cap ? ( int64_t ) n_old : d.spk_cap;
+  bool old_open = old > 0;
+  int slot_t = ( int ) ( t % d.L );
+  long long close = t - t % d.min_delay + d.min_delay;  // the open slice's end
+  na_cluster_sync();
+  if ( first && close <= end )
+    d.ctl->n_spk = 0ull;
+  while ( t < end )
+  {
+    const long long to = close < end ? close : end;
+    while ( t < to )
+    {
+      const int nk = ( int ) ( to - t < NA_LAGS ? to - t : NA_LAGS );
+      const int slot0 = slot_t;
+      double in[ NA_LAGS ];
+#pragma unroll
+      for ( int k = 0; k < NA_LAGS; ++k )
+      {
+        int slot = slot0 + k;
+        if ( slot >= d.L )
+          slot -= d.L;
+        in[ k ] = act && k < nk ? __ldcg( d.ring + ( int64_t ) slot * d.n + i ) : 0.0;
+      }
+      unsigned mask = 0;
+#pragma unroll
+      for ( int k = 0; k < NA_LAGS; ++k )
+        if ( act && k < nk )
+        {
+          double Vn = drive + P33 * V + in[ k ];
+          Vn = ( Vn < Vmin ? Vmin : Vn );
+          V = r == 0 ? Vn : V;
+          r = r == 0 ? 0 : r - 1;
+          const bool spk = V >= Vth;
+          r = spk ? refr : r;
+          V = spk ? Vreset : V;
+          mask |= ( spk ? 1u : 0u ) << k;
+        }
+#pragma unroll
+      for ( int k = 0; k < NA_LAGS; ++k )
+        if ( in[ k ] != 0.0 )
+        {
+          int slot = slot0 + k;
+          if ( slot >= d.L )
+            slot -= d.L;
+          d.ring[ ( int64_t ) slot * d.n + i ] = 0.0;
+        }
+      // the chunk's spikes: the CTA's list, the caller's output
+      int at = 0;
+      if ( mask )
+        at = atomicAdd( &s_n, __popc( mask ) );
+      __syncthreads();
+      const int n_list = s_n;
+      if ( n_list > 0 )
+      {
+        unsigned long long out0 = 0ull;
+        if ( tid == 0 )
+          out0 = atomicAdd( &d.ctl->n_out, ( unsigned long long ) n_list );
+        int q = at;
+        for ( unsigned m = mask; m; m &= m - 1 )
+          s_list[ q++ ] = ( uint32_t ) tid | ( uint32_t ) ( __ffs( m ) - 1 ) << 16;
+        __syncthreads();
+        if ( close <= end )
+        {
+          // the slice closes in this call: deliver (arrivals lie past its end)
+          for ( int k = warp; k < n_list; k += nw )
+          {
+            int slot = slot0 + ( int ) ( s_list[ k ] >> 16 );
+            if ( slot >= d.L )
+              slot -= d.L;
+            na_deliver_spike( d, ( int ) ( i0 + ( s_list[ k ] & 0xffffu ) ), slot, skipped );
+          }
+        }
+        else
+        {
+          // it stays open: a later call delivers them
+          for ( int k = tid; k < n_list; k += blockDim.x )
+          {
+            int slot = slot0 + ( int ) ( s_list[ k ] >> 16 );
+            if ( slot >= d.L )
+              slot -= d.L;
+            const unsigned long long p = atomicAdd( &d.ctl->n_spk, 1ull );
+            if ( ( int64_t ) p < d.spk_cap )
+              d.spk[ p ] = make_int2( ( int ) ( i0 + ( s_list[ k ] & 0xffffu ) ), slot );
+          }
+        }
+        if ( tid == 0 )
+          s_out = out0;
+        __syncthreads();  // (the list's last readers, too)
+        int64_t o = ( int64_t ) s_out + at;
+        for ( unsigned m = mask; m; m &= m - 1, ++o )
+          if ( o < d.out_cap )
+          {
+            d.out_src[ o ] = ( int32_t ) i;
+            d.out_stamp[ o ] = t + __ffs( m );
+          }
+        if ( tid == 0 )
+          s_n = 0;
+      }
+      __syncthreads();
+      t += nk;
+      slot_t += nk;
+      if ( slot_t >= d.L )
+        slot_t -= d.L;
+    }
+    if ( t == close )
+    {
+      if ( old_open )
+      {
+        for ( int64_t k = ( int64_t ) blockIdx.x * nw + warp; k < old; k += ( int64_t ) gridDim.x * nw )
+        {
+          const int2 sp = d.spk[ k ];
+          na_deliver_spike( d, sp.x, sp.y, skipped );
+        }
+        old_open = false;
+      }
+      close += d.min_delay;
+      na_cluster_sync();
+    }
+  }
+  if ( act )
+  {
+    d.V[ i ] = V;
+    d.r[ i ] = r;
+  }
+  if ( skipped )
+    atomicAdd( &d.ctl->n_skip, skipped );
+  na_cluster_sync();
+  if ( first )
+  {
+    *d.out_count = __ldcg( &d.ctl->n_out );
+    if ( d.out_skipped )
+      *d.out_skipped = __ldcg( &d.ctl->n_skip );
+  }
+}
+
 __global__ void
 k_na_close_slice( NaNet d )
 {
@@ -292,6 +531,35 @@ ng_simulate_noalloc( const ng_noalloc_net* net, int64_t n_steps, void* cuda_stre
   // until this call has been enqueued, no later call may continue its run
   run.valid = false;
   cudaError_t ce;
+  if ( net->n <= NA_CL_CTAS * 1024 )
+  {
+    // CTAs of 512 threads at least: their warps share the deliveries
+    const int per = ( int ) ( ( net->n + NA_CL_CTAS - 1 ) / NA_CL_CTAS );
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3( NA_CL_CTAS );
+    lc.blockDim = dim3( ( unsigned ) std::max( 512, ( per + 31 ) / 32 * 32 ) );
+    lc.stream = st;
+    cudaLaunchAttribute at[ 1 ];
+    at[ 0 ].id = cudaLaunchAttributeClusterDimension;
+    at[ 0 ].val.clusterDim.x = NA_CL_CTAS;
+    at[ 0 ].val.clusterDim.y = 1;
+    at[ 0 ].val.clusterDim.z = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    if ( cudaLaunchKernelEx( &lc, k_na_run, d, per, ( long long ) net->start_step, ( long long ) n_steps,
+           net->continue_run ? 0 : 1 )
+      != cudaSuccess )
+    {
+      ng_internal_set_error( "ng_simulate_noalloc: kernel launch failed" );
+      return NG_ERR_CUDA;
+    }
+    run.valid = true;
+    run.n = net->n;
+    run.min_delay = net->min_delay;
+    run.max_delay = net->max_delay;
+    run.next_step = net->start_step + n_steps;
+    return NG_OK;
+  }
   if ( net->continue_run )
   {
     k_na_begin_call<<< 1, 1, 0, st >>>( d );
