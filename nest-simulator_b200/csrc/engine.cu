@@ -740,7 +740,7 @@ struct ng_engine
   bool plastic_on = false;
   DevBuf pl_row, pl_tgt, pl_dly, pl_w, pl_Kplus, pl_tlast, pl_ninc, pl_tauinv, pl_Kminus, pl_last, pl_hist_t, pl_hist_K,
     pl_hist_n, pl_hist_lo, pl_drop_t, pl_drop_K, pl_nflush, pl_in_row, pl_in_edge, pl_in_src, pl_wrun, pl_tab_fin,
-    pl_tab_km;
+    pl_tab_km, pl_list, pl_items, pl_spk, pl_done, pl_fitems;
   int64_t pl_nnz = 0, pl_nsrc = 0;
   double pl_dmax_ms = 0;
   int32_t pl_dconst = -1;  // the plastic delay when all are equal
@@ -808,7 +808,7 @@ struct ng_engine
       &net_spk, &log_sorted, &log_cnt, &log_off, &sc_bound, &seg, &net_t, &row_ue, &row_ls, &ent_late, &pk, &pl_row,
       &pl_tgt, &pl_dly, &pl_w, &pl_Kplus, &pl_tlast, &pl_ninc, &pl_tauinv, &pl_Kminus, &pl_last, &pl_hist_t, &pl_hist_K,
       &pl_hist_n, &pl_hist_lo, &pl_drop_t, &pl_drop_K, &pl_nflush, &pl_in_row, &pl_in_edge, &pl_in_src, &pl_wrun,
-      &pl_tab_fin, &pl_tab_km, &own_cta, &own_rpb, &own_rp, &own_eb, &own_rpf, &own_ebf, &own_word, &own_weight, &own_x };
+      &pl_tab_fin, &pl_tab_km, &pl_list, &pl_items, &pl_spk, &pl_done, &pl_fitems, &own_cta, &own_rpb, &own_rp, &own_eb, &own_rpf, &own_ebf, &own_word, &own_weight, &own_x };
     for ( DevBuf* b : bufs )
       cudaFree( b->p );
     if ( host_ctl )
@@ -1162,9 +1162,9 @@ struct ng_engine
     const int span = to_ - from_;
     // the tuned (or default) kernel; one thread per neuron for 1-2 step
     // slices and for engines with the per-target gather or the target-tiled
-    // delivery (the lag bits are written there)
+    // delivery (the network's mode and spike count are kept there)
     int v = upd_variant >= 0 ? upd_variant : engine_default_variant( db.n );
-    if ( span <= 2 || gather_on || tiled_on || plastic_on )
+    if ( span <= 2 || gather_on || tiled_on )
       v = ( v == 1 || v == 6 ) ? v : 0;
     if ( v <= 1 || v == 6 )
     {
@@ -1731,6 +1731,11 @@ struct ng_engine
     p.in_src = ( const int32_t* ) pl_in_src.p;
     p.dmax_ms = pl_dmax_ms;
     p.dconst = pl_dconst;
+    p.n_list = ( int32_t* ) pl_list.p;
+    p.items = ( int4* ) pl_items.p;
+    p.fl_items = ( int2* ) pl_fitems.p;
+    p.n_done = ( int32_t* ) pl_done.p;
+    p.spk = ( StdpSpike* ) pl_spk.p;
     p.tab_fin = ( int32_t* ) pl_tab_fin.p;
     p.tab_km = ( double* ) pl_tab_km.p;
     p.lambda = pl_lambda;
@@ -1752,19 +1757,21 @@ struct ng_engine
       // read only earlier slices' postsynaptic spikes), then the histories
       const StdpNet p = stdp();
       const unsigned ga = ( unsigned ) std::max< int64_t >( 1, std::min< int64_t >( ( N + 255 ) / 256, 4 * sms ) );
-      const unsigned gd = ( unsigned ) std::max< int64_t >( 1, std::min< int64_t >( pl_nsrc, 8 * sms ) );
       if ( pl_dconst >= 0 )
       {
         const int64_t q = N * cfg.min_delay;
         k_stdp_arrivals<<< ( unsigned ) std::max< int64_t >( 1, std::min< int64_t >( ( q + 255 ) / 256, 8 * sms ) ), 256, 0,
           stream >>>( d, p );
       }
+      k_stdp_spikes<<< ( unsigned ) std::max< int64_t >( 1, std::min< int64_t >( ( pl_nsrc + 255 ) / 256, 4 * sms ) ), 256, 0,
+        stream >>>( d, p );
+      const unsigned gd = ( unsigned ) ( 4 * sms );
       if ( prec == NG_FP64 )
-        k_stdp_deliver< false ><<< gd, 256, 0, stream >>>( d, p );
+        k_stdp_deliver< false ><<< gd, STDP_CHUNK, 0, stream >>>( d, p );
       else
-        k_stdp_deliver< true ><<< gd, 256, 0, stream >>>( d, p );
+        k_stdp_deliver< true ><<< gd, STDP_CHUNK, 0, stream >>>( d, p );
       k_stdp_archive<<< ga, 256, 0, stream >>>( d, p );
-      k_stdp_flush<<< ( unsigned ) std::max< int64_t >( 1, std::min< int64_t >( N, 8 * sms ) ), 256, 0, stream >>>( d, p );
+      k_stdp_flush<<< ( unsigned ) ( 4 * sms ), STDP_CHUNK, 0, stream >>>( d, p );
     }
     if ( gather_live )
       k_gather<<< ( unsigned ) sms, G_THREADS, G_SMEM, stream >>>( d );
@@ -2474,7 +2481,7 @@ struct ng_engine
     if ( iaf )
     {
       variants = { 0, 1, 6 };
-      if ( md >= 3 && !gather_on && !tiled_on && !plastic_on )
+      if ( md >= 3 && !gather_on && !tiled_on )
       {
         variants.push_back( 2 );
         variants.push_back( 3 );
@@ -3339,6 +3346,11 @@ ng_set_plastic_connections( ng_engine* e, int64_t n_src, const int64_t* row_ptr,
     || ( rc = e->upload( e->pl_in_src, in_src.data(), in_src.size() * 4 ) ) )
     return rc;
   if ( !e->gmask.p && ( rc = e->alloc( e->gmask, N * 4 ) ) )
+    return rc;
+  if ( ( rc = e->alloc( e->pl_list, 16 ) ) || ( rc = e->alloc( e->pl_done, N * 4 ) )
+    || ( rc = e->alloc( e->pl_fitems, ( ( size_t ) nnz / STDP_CHUNK + N + 1 ) * sizeof( int2 ) ) )
+    || ( rc = e->alloc( e->pl_items, ( ( size_t ) nnz / STDP_CHUNK + ( size_t ) n_src + 1 ) * sizeof( int4 ) ) )
+    || ( rc = e->alloc( e->pl_spk, std::max< size_t >( ( size_t ) n_src, 1 ) * ( size_t ) e->cfg.min_delay * sizeof( StdpSpike ) ) ) )
     return rc;
   if ( e->pl_dconst >= 0 )
   {

@@ -1255,6 +1255,14 @@ k_update_iaf2( Net d, Block b, int from, int to, int sched )
         if ( ++slot == d.L )
           slot = 0;
       }
+      if ( d.gmask && act )
+      {
+        // lag bits of the slice for the plastic connections (min_delay <= 32)
+        if ( cb == 0 )
+          d.gmask[ i ] = smask;
+        else
+          d.gmask[ i ] |= smask << cb;
+      }
       warp_append_mask( d, smask, ( int32_t ) i, slot0, t0 );
     }
     __syncthreads();

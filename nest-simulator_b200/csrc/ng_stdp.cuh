@@ -8,14 +8,17 @@
 // connection of one source -- all start at 0 and see the same presynaptic
 // spikes -- so they are kept per source.  At the close of a slice, after the
 // node update has set each neuron's lag bits of the slice (gmask):
-//   k_stdp_deliver  one CTA per spiking source splits its plastic row; each
+//   k_stdp_spikes   lists the spiking sources and lays out each one's spikes of
+//                   the slice with the Kplus and t_last before them, then
+//                   advances the source's Kplus and t_last;
+//   k_stdp_deliver  one CTA per chunk of a spiking source's plastic row; each
 //                   thread applies the source's spikes of the slice to its
 //                   connections in time order: facilitation by the target's
 //                   history entries in (t_last - d, t_spike - d], depression by
 //                   the target's trace at t_spike - d, the new weight into the
-//                   ring buffer (stdp_pl_synapse_hom::send, :255-298); then the
-//                   source's Kplus and t_last.  The slice's own postsynaptic
-//                   spikes are never read here: t_spike - d <= the slice origin.
+//                   ring buffer (stdp_pl_synapse_hom::send, :255-298).  The
+//                   slice's own postsynaptic spikes are never read here:
+//                   t_spike - d <= the slice origin.
 //   k_stdp_archive  appends every postsynaptic spike of the slice to its
 //                   neuron's history (time, Kminus trace), in time order
 //                   (ArchivingNode::set_spiketime, archiving_node.cpp:182-220),
@@ -45,9 +48,17 @@ namespace ng
 {
 
 constexpr int STDP_HIST = 64;
+constexpr int STDP_CHUNK = 256;      // connections of a delivery item, one per thread
 constexpr int STDP_KEEP = 16;        // entries a flush leaves in the ring
 constexpr int ERR_STDP_HISTORY = 32;
 constexpr double STDP_EPS = 1.0e-6;  // ConnectionManager's stdp_eps default
+
+// A spike of a listed source, with the source's trace before it.
+struct StdpSpike
+{
+  double t, Kplus, tlast;  // time [ms], Kplus and t_last before the spike
+  int k, slot;             // lag, ring slot of the emission
+};
 
 struct StdpNet
 {
@@ -70,6 +81,7 @@ struct StdpNet
   double* drop_t;         // per neuron: newest dropped entry (time, Kminus)
   double* drop_K;
   int32_t* n_flush;       // per neuron: entries the next flush drops
+  int32_t* n_done;        // per neuron: items of its flush that are done
   const int64_t* in_row;  // per neuron: its incoming plastic connections (N + 1)
   const uint32_t* in_edge;  // their indices in the CSR
   const int32_t* in_src;
@@ -77,6 +89,11 @@ struct StdpNet
   int32_t dconst;         // the plastic delay in steps when all are equal, else -1
   int32_t* tab_fin;       // dconst >= 0: per (neuron, lag of the slice) the end of the
   double* tab_km;         //   facilitation range and the depression trace (k_stdp_arrivals)
+  int32_t* n_list;        // spiking sources of the slice, delivery items (reset by k_stdp_archive), flush
+                          // items (reset by k_stdp_spikes)
+  int2* fl_items;         // flush items: neuron, first incoming connection
+  int4* items;            // delivery items: source, its place among the spiking ones, first connection
+  StdpSpike* spk;         // [place][min_delay]
   double lambda, alpha, mu, tau_plus_inv;
   double ms_per_tic;      // Time::get_ms = MS_PER_TIC * tics
   int64_t tics_per_step;
@@ -93,6 +110,8 @@ __global__ void
 k_stdp_archive( Net d, StdpNet p )
 {
   const long long origin = cta_origin( d );
+  if ( blockIdx.x == 0 && threadIdx.x == 0 )
+    p.n_list[ 0 ] = p.n_list[ 1 ] = 0;  // (behind the slice's delivery)
   for ( int64_t i = ( int64_t ) blockIdx.x * blockDim.x + threadIdx.x; i < d.N; i += ( int64_t ) gridDim.x * blockDim.x )
   {
     if ( !p.n_inc[ i ] )
@@ -129,7 +148,15 @@ k_stdp_archive( Net d, StdpNet p )
         ++k;
       if ( hn - k > STDP_HIST - 32 )
         atomicOr( &d.ctl->err, ERR_STDP_HISTORY );
-      p.n_flush[ i ] = ( int32_t ) ( k - lo );
+      if ( k > lo )
+      {
+        p.n_flush[ i ] = ( int32_t ) ( k - lo );
+        const int64_t deg = p.in_row[ i + 1 ] - p.in_row[ i ];
+        const int chunks = ( int ) ( ( deg + STDP_CHUNK - 1 ) / STDP_CHUNK );
+        const int at = atomicAdd( p.n_list + 2, chunks );
+        for ( int c = 0; c < chunks; ++c )
+          p.fl_items[ at + c ] = make_int2( ( int ) i, c * STDP_CHUNK );
+      }
     }
   }
 }
@@ -238,18 +265,24 @@ k_stdp_arrivals( Net d, StdpNet p )
 // applies the facilitation of those in its current window (t >= t_last - d
 // + eps; later bounds hold since the entries arrived before the slice's
 // end), in time order, with its source's Kplus and t_last.
-__global__ void __launch_bounds__( 256 )
+// One CTA per item, a chunk of a neuron's incoming connections (ten neurons
+// flush in a slice of 4,500; a CTA for each ran a thread through seven
+// connections of sixteen terms: 48 us per slice, in chunks 10 us); the last
+// item of a neuron drops the entries.
+__global__ void __launch_bounds__( STDP_CHUNK )
 k_stdp_flush( Net d, StdpNet p )
 {
-  for ( int64_t tg = blockIdx.x; tg < d.N; tg += gridDim.x )
+  const int n_items = p.n_list[ 2 ];
+  for ( int item = blockIdx.x; item < n_items; item += gridDim.x )
   {
+    const int2 it = p.fl_items[ item ];
+    const int tg = it.x;
     const int nf = p.n_flush[ tg ];
-    if ( nf == 0 )
-      continue;  // uniform over the CTA
     const int64_t lo = p.hist_lo[ tg ];
-    const double* ht = p.hist_t + tg * STDP_HIST;
+    const double* ht = p.hist_t + ( int64_t ) tg * STDP_HIST;
     const int64_t i0 = p.in_row[ tg ], i1 = p.in_row[ tg + 1 ];
-    for ( int64_t q = i0 + threadIdx.x; q < i1; q += blockDim.x )
+    const int64_t q = i0 + it.y + threadIdx.x;
+    if ( q < i1 )
     {
       const uint32_t e = p.in_edge[ q ];
       const int32_t src = p.in_src[ q ];
@@ -273,70 +306,86 @@ k_stdp_flush( Net d, StdpNet p )
     __syncthreads();
     if ( threadIdx.x == 0 )
     {
-      const int64_t last = ( lo + nf - 1 ) % STDP_HIST;
-      p.drop_t[ tg ] = ht[ last ];
-      p.drop_K[ tg ] = p.hist_K[ tg * STDP_HIST + last ];
-      p.hist_lo[ tg ] = lo + nf;
-      p.n_flush[ tg ] = 0;
+      const int chunks = ( int ) ( ( i1 - i0 + STDP_CHUNK - 1 ) / STDP_CHUNK );
+      __threadfence();  // (the other items have read lo and n_flush before their count)
+      if ( atomicAdd( p.n_done + tg, 1 ) == chunks - 1 )
+      {
+        const int64_t last = ( lo + nf - 1 ) % STDP_HIST;
+        p.drop_t[ tg ] = ht[ last ];
+        p.drop_K[ tg ] = p.hist_K[ ( int64_t ) tg * STDP_HIST + last ];
+        p.hist_lo[ tg ] = lo + nf;
+        p.n_flush[ tg ] = 0;
+        p.n_done[ tg ] = 0;
+      }
     }
   }
 }
 
-// One CTA per spiking source at a time (grid-stride over sources): the
-// CTA's threads split the source's plastic row, so a spike's thousands of
-// connections -- each a chain of dependent history loads -- run on 256
-// threads instead of 32.  Thread 0 first lays out the source's spikes of
-// the slice in shared memory (lag, time, ring slot, and Kplus / t_last
-// before each spike) and advances the source's Kplus and t_last; each
-// thread then applies the spikes to its connections in time order.
+__global__ void
+k_stdp_spikes( Net d, StdpNet p )
+{
+  const long long origin = cta_origin( d );
+  if ( blockIdx.x == 0 && threadIdx.x == 0 )
+    p.n_list[ 2 ] = 0;
+  unsigned long long events = 0;
+  for ( int64_t src = ( int64_t ) blockIdx.x * blockDim.x + threadIdx.x; src < p.n_src;
+        src += ( int64_t ) gridDim.x * blockDim.x )
+  {
+    unsigned m = d.gmask[ src ];
+    const int64_t deg = p.row[ src + 1 ] - p.row[ src ];
+    if ( m == 0 || deg == 0 )
+      continue;
+    const int at = atomicAdd( p.n_list, 1 );
+    const int chunks = ( int ) ( ( deg + STDP_CHUNK - 1 ) / STDP_CHUNK );
+    const int it = atomicAdd( p.n_list + 1, chunks );
+    for ( int c = 0; c < chunks; ++c )
+      p.items[ it + c ] = make_int4( ( int ) src, at, c * STDP_CHUNK, __popc( m ) );
+    StdpSpike* const s = p.spk + ( int64_t ) at * d.min_delay;
+    double Kp = p.Kplus[ src ], tl = p.tlast[ src ];
+    for ( int n = 0; m; m &= m - 1, ++n )
+    {
+      const int k = __ffs( m ) - 1;
+      const double t_spike = stdp_stamp_ms( p, origin + k + 1 );
+      s[ n ] = StdpSpike { t_spike, Kp, tl, k, ( int ) ( ( origin + k ) % d.L ) };
+      Kp = Kp * exp( ( tl - t_spike ) * p.tau_plus_inv ) + 1.0;
+      tl = t_spike;
+      events += ( unsigned long long ) deg;
+    }
+    p.Kplus[ src ] = Kp;
+    p.tlast[ src ] = tl;
+  }
+  if ( events )
+    atomicAdd( &d.ctl->syn_events, events );
+}
+
+// One CTA per item: STDP_CHUNK connections of a spiking source, one per
+// thread.  A slice has one or two hundred spiking
+// sources of thousands of connections: a CTA per source left most of the
+// chip's CTA slots empty and ran a thread through seven connections, a chain
+// of dependent history loads, exponentials and logarithms each (61 us per
+// slice of 124 sources x 1,800 connections; in chunks 21 us).
 // (registers capped for four CTAs per SM: more resident warps hide the
 // dependent history loads better than spill-free code -- measured RTF 0.407
 // against 0.424 with 80 registers, 0.420 with 48 on the hpc_benchmark network)
 template < bool FIX >
-__global__ void __launch_bounds__( 256, 4 )
+__global__ void __launch_bounds__( STDP_CHUNK, 4 )
 k_stdp_deliver( Net d, StdpNet p )
 {
-  __shared__ double s_t[ 32 ], s_Kp[ 32 ], s_tl[ 32 ];
-  __shared__ int s_k[ 32 ], s_slot0[ 32 ];
-  __shared__ int s_n;
-  const long long origin = cta_origin( d );
+  __shared__ StdpSpike s_spk[ 32 ];
   const double h_ms = p.ms_per_tic * ( double ) p.tics_per_step;
   const int md = d.min_delay;
+  const int n_items = p.n_list[ 1 ];
   bool overflow = false;
-  unsigned long long events = 0;
-  for ( int64_t src = blockIdx.x; src < p.n_src; src += gridDim.x )
+  for ( int item = blockIdx.x; item < n_items; item += gridDim.x )
   {
-    const unsigned m0 = d.gmask[ src ];
-    const int64_t e0 = p.row[ src ], e1 = p.row[ src + 1 ];
-    if ( m0 == 0 || e1 == e0 )
-      continue;  // uniform over the CTA
-    if ( threadIdx.x == 0 )
-    {
-      double Kp = p.Kplus[ src ], tl = p.tlast[ src ];
-      int n = 0;
-      unsigned m = m0;
-      while ( m )
-      {
-        const int k = __ffs( m ) - 1;
-        m &= m - 1;
-        const double t_spike = stdp_stamp_ms( p, origin + k + 1 );
-        s_k[ n ] = k;
-        s_t[ n ] = t_spike;
-        s_Kp[ n ] = Kp;
-        s_tl[ n ] = tl;
-        s_slot0[ n ] = ( int ) ( ( origin + k ) % d.L );
-        Kp = Kp * exp( ( tl - t_spike ) * p.tau_plus_inv ) + 1.0;
-        tl = t_spike;
-        ++n;
-      }
-      s_n = n;
-      p.Kplus[ src ] = Kp;
-      p.tlast[ src ] = tl;
-      events += ( unsigned long long ) ( e1 - e0 ) * ( unsigned long long ) n;
-    }
+    const int4 it = p.items[ item ];
+    const int ns = it.w;
+    __syncthreads();  // the table's last readers
+    if ( threadIdx.x < ns )
+      s_spk[ threadIdx.x ] = p.spk[ ( int64_t ) it.y * md + threadIdx.x ];
     __syncthreads();
-    const int ns = s_n;
-    for ( int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x )
+    const int64_t e = p.row[ it.x ] + it.z + threadIdx.x;
+    if ( e < p.row[ it.x + 1 ] )
     {
       const int32_t tg = p.tgt[ e ];
       const int32_t dl = p.dconst >= 0 ? p.dconst : p.dly[ e ];
@@ -347,23 +396,24 @@ k_stdp_deliver( Net d, StdpNet p )
       const double* ht = p.hist_t + ( int64_t ) tg * STDP_HIST;
       for ( int j = 0; j < ns; ++j )
       {
+        const StdpSpike& sp = s_spk[ j ];
         int64_t fin;
         double kminus;
         if ( p.dconst >= 0 )
         {
-          const int64_t q = ( int64_t ) tg * md + s_k[ j ];
+          const int64_t q = ( int64_t ) tg * md + sp.k;
           fin = lo + p.tab_fin[ q ];
           kminus = p.tab_km[ q ];
         }
         else
         {
-          const double t = s_t[ j ] - d_ms;
+          const double t = sp.t - d_ms;
           fin = stdp_fin( ht, lo, hn, t );
           kminus = stdp_kminus( p, tg, ht, p.hist_K + ( int64_t ) tg * STDP_HIST, lo, fin, t, overflow );
         }
-        w = stdp_pl_apply( p, ht, lo, fin, w, d_ms, s_Kp[ j ], s_tl[ j ], kminus );
+        w = stdp_pl_apply( p, ht, lo, fin, w, d_ms, sp.Kplus, sp.tlast, kminus );
         // handle(SpikeEvent&): weight x multiplicity into the channel of its sign
-        int slot = s_slot0[ j ] + dl;
+        int slot = sp.slot + dl;
         if ( slot >= d.L )
           slot -= d.L;
         const int ch = ( p.sign_channels && !( w > 0.0 ) ) ? 1 : 0;
@@ -377,10 +427,7 @@ k_stdp_deliver( Net d, StdpNet p )
       p.w[ e ] = w;
       p.w_run[ e ] = w;
     }
-    __syncthreads();  // the spike table is rewritten for the next source
   }
-  if ( threadIdx.x == 0 && events )
-    atomicAdd( &d.ctl->syn_events, events );
   if ( overflow )
     atomicOr( &d.ctl->err, ERR_STDP_HISTORY );
 }
