@@ -264,7 +264,8 @@ int ng_set_graph_slices( ng_engine* eng, int32_t slices_per_graph );
 typedef struct
 {
   int32_t mode;            /* 0: fixed, 1: autotuned */
-  int32_t state;           /* 0: not tuned yet, 1: measured, 2: from the process cache, 3: fixed */
+  int32_t state;           /* 0: not tuned yet, 1: measured (without trials below: chosen by rule), 2: from
+                              the process cache, 3: fixed */
   int32_t update_variant;  /* 0/1/6: one thread per neuron (4/8/2 lags of inputs at a time), 2/3:
                               two-phase (256/128-thread CTAs), 4: aeif_cond_alpha's RKF45 kernel,
                               5: the persistent slice kernels (the target-owning one where the

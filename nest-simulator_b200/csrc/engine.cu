@@ -2574,6 +2574,22 @@ struct ng_engine
         return NG_OK;
       }
     }
+    // A static network that k_run_owned takes runs in it without trials (a
+    // serving engine, tuned on request only, measures).  It was the
+    // fastest form of every such network measured, from 100 neurons of 12
+    // inputs to 150,000 of 60 (one call of 1 s or 0.6 s, it against the best
+    // of the others [ms]: 100 x 12 3.2 / 8.7, 20,000 x 60 10.5 / 20.1, 20,000 x
+    // 200 9.9 / 18.5, 100,000 x 100 32.9 / 44.5, 100,000 x 1,000 15.1 / 26.5,
+    // 150,000 x 60 56.9 / 67.1), and trials of few steps can choose wrongly:
+    // in the layered network of 77,169 neurons, which alternates between
+    // silence and bursts, a group of 9 steps took from 29 to 190 us per step
+    // with one and the same form.
+    if ( tune_mode == 1 && !serving && own_ready() )
+    {
+      apply_cand( TuneCand { 5, deliver_per_sm, deliver_group, 0.0 } );
+      tune_state = 1;
+      return NG_OK;
+    }
     auto trial = [ & ]( TuneCand c, double* us ) -> int {
       apply_cand( c );
       double warm = 0;

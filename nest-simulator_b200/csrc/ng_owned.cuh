@@ -38,6 +38,18 @@
 // global ring cell, which the update adds in.  The edges whose delay can
 // exceed the window are segments of their own, so that the others are added
 // without a look at it.
+//
+// What bounds it.  Small and middle networks: a slice is one chain (inputs
+// 1.4k cycles, recurrence beside the drive 2-3.5k, exchange 3.5-4k, delivery
+// 2k: 10-12k cycles on 9,000 to 12,500 neurons).  Large ones: the segments'
+// random reads (77,169 neurons: 72k of 112k cycles a step, 1,580 spikes of
+// some 26 edges per SM; 1,569 segments of 320 B alone take 37k cycles, 3.8
+// TB/s) beside the adds (32-bit shared atomics: 2.5 cycles per random warp
+// instruction; 64-bit ones 18).  One call, the scatter or graph form before
+// and this kernel [us]: 10,000 steps of 12,500 neurons in FP64 9,283 -> 6,234,
+// of 9,377 in FP32 8,773 -> 5,610; 5,000 steps of 8 x 7,001 neurons 16,085 ->
+// 8,471; 300 steps of the layered network at 1/4 size in FP64 8,626 -> 3,741,
+// at full size in FP32 30,113 -> 17,636.
 #pragma once
 
 #include "ng_persistent.cuh"
@@ -54,7 +66,7 @@ enum
 
 constexpr int OW_LIST = 4096;        // spikes staged in shared memory at a time
 constexpr int OW_TAB = 64;           // OW_COUNT: inputs of up to OW_TAB - 1 events of a class, tabulated
-constexpr int OW_TPB = 512;          // threads per CTA (16 warps of up to 128 registers, no spills)
+constexpr int OW_TPB = 512;          // threads per CTA: 16 warps of up to 128 registers (1024 spilled 350-800 B a thread)
 constexpr int OW_DVT = 32;           // drive inputs tabulated where a CTA's neurons share one weight
 constexpr int OW_MAX_G = 256;        // CTAs of a network, at most
 constexpr int OW_CDF = 512;          // drive thresholds staged in shared memory (more: read through L1)

@@ -225,7 +225,7 @@ k_na_run( NaNet d, int per, long long start, long long n_steps, int fresh )
   __shared__ uint32_t s_list[ NA_LIST ];  // local neuron, lag of the chunk << 16
   __shared__ int s_n;
   __shared__ unsigned long long s_out;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, nw = blockDim.x >> 5;
   const int64_t i0 = ( int64_t ) blockIdx.x * per, i = i0 + tid;  // `per` neurons per CTA
   const bool act = tid < per && i < d.n;
   const bool first = blockIdx.x == 0 && tid == 0;

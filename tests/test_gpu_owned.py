@@ -34,7 +34,8 @@ def _run(variant, precision, model, n, copies, deg, md, maxd, uniform, hot, trac
     if model == DELTA:
         w = w / 256.0
     eng = _abi.Engine([(model, N)], 0.1, md, maxd, precision=precision)
-    eng.set_tuning(0, variant, -1, -1)
+    if variant >= 0:
+        eng.set_tuning(0, variant, -1, -1)
     eng.set_var(0, "V_m_rel", np.full(N, 16.0) if hot else rng.uniform(0.0, 14.5, N))
     eng.set_connections(row, tgt.astype(np.int32), w, rng.integers(md, maxd + 1, nnz).astype(np.int32))
     eng.set_recording((np.arange(N) % 7 != 3).astype(np.uint8))
@@ -50,9 +51,9 @@ def _run(variant, precision, model, n, copies, deg, md, maxd, uniform, hot, trac
     out = [s[o], t[o]] + [eng.get_var(0, v) for v in (("V_m_rel",) if model == DELTA else ("V_m_rel", "I_syn_ex", "I_syn_in"))]
     if trace:
         out.append(eng.trace()[1])
-    st = eng.stats()
+    st, tuned = eng.stats(), eng.tuned()
     eng.close()
-    return out, (st["spikes"], st["syn_events"], st["drive_events"]), st["update_launches"]
+    return out, (st["spikes"], st["syn_events"], st["drive_events"]), st["update_launches"], tuned
 
 
 CASES = [
@@ -74,11 +75,24 @@ CASES = [
 
 @pytest.mark.parametrize("case", CASES)
 def test_owned_equals_graph_form(case):
-    ref, st0, _ = _run(0, *case)
-    got, st1, launches = _run(5, *case)
+    ref, st0 = _run(0, *case)[:2]
+    got, st1, launches, _ = _run(5, *case)
     assert len(ref[0]) > 20
     assert st0 == st1
     for a, b in zip(got, ref):
         np.testing.assert_array_equal(a, b)
     # full slices ran many to a launch
     assert launches < sum(case[-1]) // case[5] + len(case[-1])
+
+
+@pytest.mark.parametrize("md", [1, 15])
+def test_default_mode_takes_it_without_trials(md):
+    # a network no other test has (the process keeps what was measured), in
+    # one call long enough for every trial
+    case = (_abi.NG_FP64, EXP, 2111 + md, 1, 33, md, 15, False, False, False, (4000 if md > 1 else 600,))
+    ref, st0 = _run(0, *case)[:2]
+    got, st1, _, tuned = _run(-1, *case)
+    assert st0 == st1
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
+    assert tuned["state"] == "tuned" and tuned["update_variant"] == 5 and not tuned["candidates"]
