@@ -43,7 +43,7 @@
 // 1.4k cycles, recurrence beside the drive 2-3.5k, exchange 3.5-4k, delivery
 // 2k: 10-12k cycles on 9,000 to 12,500 neurons).  Large ones: the segments'
 // random reads (77,169 neurons: 72k of 112k cycles a step, 1,580 spikes of
-// some 26 edges per SM; 1,569 segments of 320 B alone take 37k cycles, 3.8
+// some 40 edges per SM; 1,569 segments of 320 B alone take 37k cycles, 3.8
 // TB/s) beside the adds (32-bit shared atomics: 2.5 cycles per random warp
 // instruction; 64-bit ones 18).  One call, the scatter or graph form before
 // and this kernel [us]: 10,000 steps of 12,500 neurons in FP64 9,283 -> 6,234,
