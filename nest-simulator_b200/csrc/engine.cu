@@ -1189,7 +1189,7 @@ struct ng_engine
     // the tuned (or default) kernel; one thread per neuron for 1-2 step
     // slices and for engines with the per-target gather or the target-tiled
     // delivery (the network's mode and spike count are kept there)
-    int v = upd_variant >= 0 ? upd_variant : engine_default_variant( db.n );
+    int v = upd_variant >= 0 && upd_variant != 5 ? upd_variant : engine_default_variant( db.n );
     if ( span <= 2 || gather_on || tiled_on )
       v = ( v == 1 || v == 6 ) ? v : 0;
     if ( v <= 1 || v == 6 )
@@ -1993,11 +1993,15 @@ struct ng_engine
     while ( n > 0 )
     {
       // the persistent forms: the target-owning kernel where the network
-      // suits it -- also before tuning, from two slices on -- else the
-      // scatter form
+      // suits it -- also before tuning -- else the scatter form.  A single
+      // slice (a node's call per slice) does not repay the owning kernel's
+      // prologue and epilogue: 43 against 21 us per call at 12,500 neurons
+      // (one-wave scatter form), 54 against 25 at 19,300 (graph).
       const int64_t full = from == 0 ? n / cfg.min_delay : 0;
-      const int64_t owned = upd_variant == 5 || ( upd_variant < 0 && full > 1 ) ? own_slices( full ) : 0;
-      if ( full > 0 && ( owned > 0 || ( upd_variant == 5 && persistent_ok() ) ) )
+      const int64_t owned = ( upd_variant == 5 || upd_variant < 0 ) && full > 1 ? own_slices( full ) : 0;
+      const bool scatter = owned == 0 && upd_variant == 5 && full > 0 && persistent_ok()
+        && ( full > 1 || !pk_multi_group() || !own_ready() );
+      if ( owned > 0 || scatter )
       {
         const int k = ( int ) std::min< int64_t >( owned > 0 ? owned : full, 1 << 20 );
         late_join();

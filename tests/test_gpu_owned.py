@@ -96,3 +96,13 @@ def test_default_mode_takes_it_without_trials(md):
     for a, b in zip(got, ref):
         np.testing.assert_array_equal(a, b)
     assert tuned["state"] == "tuned" and tuned["update_variant"] == 5 and not tuned["candidates"]
+
+
+def test_single_slices_after_many():
+    # calls of one slice take another form than the calls of many around them
+    case = (_abi.NG_FP64, EXP, 15011, 1, 20, 5, 12, False, False, False, (200, 5, 5, 5, 3, 2, 5, 60))
+    ref, st0 = _run(0, *case)[:2]
+    got, st1 = _run(5, *case)[:2]
+    assert len(ref[0]) > 20 and st0 == st1
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
