@@ -1270,6 +1270,21 @@ struct ng_engine
     return N > ( int64_t ) pk_occ * sms * PK_NB;
   }
 
+  // A kernel's dynamic shared memory limit belongs to the function, for the
+  // whole process: an engine that set it to its own layout's size would lower
+  // it under another engine's launches.  Every engine sets it to the most the
+  // device allows beside the kernel's static part, the same value from all.
+  int
+  max_dynamic_smem( const void* func )
+  {
+    cudaFuncAttributes fa;
+    int optin = 0;
+    CU( cudaFuncGetAttributes( &fa, func ) );
+    CU( cudaDeviceGetAttribute( &optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg.device ) );
+    CU( cudaFuncSetAttribute( func, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - ( int ) fa.sharedSizeBytes ) );
+    return NG_OK;
+  }
+
   // ---- target-owning slice kernel
   template < typename Real, bool FIX, int MODEL, int CELL >
   const void*
@@ -1595,8 +1610,8 @@ struct ng_engine
       } );
     }
     CU( cudaGetLastError() );
-    CU( cudaFuncSetAttribute( own_kernel( cell, own_held ), cudaFuncAttributeMaxDynamicSharedMemorySize,
-      ( int ) own_smem_bytes ) );
+    if ( ( rc = max_dynamic_smem( own_kernel( cell, own_held ) ) ) )
+      return rc;
     int occ = 0, coop = 0;
     CU( cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, cfg.device ) );
     CU( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, own_kernel( cell, own_held ), OW_TPB, own_smem_bytes ) );
