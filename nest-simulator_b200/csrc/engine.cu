@@ -604,17 +604,10 @@ struct ng_engine
       {
         tiled_on = true;
         tile_smem = W * C * tile_t * esz;
-        cudaError_t ce;
-        if ( prec == NG_FP64 )
-          ce = cudaFuncSetAttribute( k_deliver_tiled< double, false >, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            ( int ) tile_smem );
-        else if ( ring_bytes == 4 )
-          ce = cudaFuncSetAttribute( k_deliver_tiled< int32_t, true >, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            ( int ) tile_smem );
-        else
-          ce = cudaFuncSetAttribute( k_deliver_tiled< long long, true >, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            ( int ) tile_smem );
-        if ( ce != cudaSuccess )
+        const void* const func = prec == NG_FP64 ? reinterpret_cast< const void* >( &k_deliver_tiled< double, false > )
+          : ring_bytes == 4 ? reinterpret_cast< const void* >( &k_deliver_tiled< int32_t, true > )
+                            : reinterpret_cast< const void* >( &k_deliver_tiled< long long, true > );
+        if ( max_dynamic_smem( func ) != NG_OK )
           return fail( NG_ERR_CUDA, "serving: cannot reserve shared memory for the tiled delivery" );
         if ( ( rc = alloc( seg, ( size_t ) cfg.tile_capacity * 4 ) )
           || ( rc = alloc( net_t, ( size_t ) nmax * sizeof( TileNet ) ) ) )

@@ -1,7 +1,8 @@
-"""Engines of one process whose networks run in the target-owning slice kernel
-with layouts of different sizes: what one engine sets up must not reach
-another.  Weights and drive are dyadic, so each engine's results equal, bit
-for bit, those of the same network run alone."""
+"""Engines of one process whose kernels (the target-owning slice kernel, the
+target-tiled delivery) have layouts of different sizes: what one engine sets
+up must not reach another.  Weights and drive are dyadic (or the form is fixed
+point), so each engine's results equal, bit for bit, those of the same network
+run alone."""
 
 import threading
 
@@ -9,6 +10,8 @@ import numpy as np
 import pytest
 
 from nestgpu import _abi
+
+from test_gpu_serving import PB_SIZES, _pb
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +89,30 @@ def test_engines_on_two_threads():
     assert not failed
     for e, w in zip(engines, want):
         _assert_same(_result(e), w)
+
+
+def test_tiled_engines():
+    """The second engine's shorter delays give its tiles a smaller window."""
+    n = sum(PB_SIZES)
+
+    def engine(max_delay):
+        return _abi.Engine([(_abi.NG_IAF_PSC_EXP, 20_000)], 0.1, 1, max_delay, precision=_abi.NG_FP32, serving=True,
+                           max_networks=2, edge_capacity=30_000_000, max_abs_weight=1000.0,
+                           tile_capacity=_abi.tile_table_entries(n, max_delay, False))
+
+    def run(with_other):
+        eng = engine(40)
+        V0 = np.random.default_rng(8).uniform(0.0, 14.0, n)
+        nid = eng.net_add(n, 600, 17, {"tau_syn_ex": 0.5, "tau_syn_in": 0.5, "V_m_rel": V0}, build=_pb(seed=21),
+                          poisson=(np.full(n, 9000.0), 87.8, 15))
+        other = engine(3) if with_other else None
+        eng.simulate(600)
+        s, t = eng.net_spikes(nid)
+        o = np.lexsort((s, t))
+        out = s[o], t[o], eng.net_get_var(nid, "V_m_rel", n)
+        eng.close()
+        if other:
+            other.close()
+        return out
+
+    _assert_same(run(False), run(True))
