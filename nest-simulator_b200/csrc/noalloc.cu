@@ -160,21 +160,29 @@ k_na_deliver( NaNet d )
 }
 
 // ---------------------------------------------------------------------
-// A call on a network of up to NA_CL_CTAS x 1024 neurons in one launch: one
+// A call on a network of up to NA_CL_CTAS x NA_CL_TPB neurons in one launch: one
 // cluster of CTAs, one thread per neuron.  A CTA keeps its neurons' state in
 // registers and its own spikes of the open slice in shared memory, delivers
 // them itself when the slice closes (the ring holds min_delay + max_delay
 // slots, so a delivery meets no cell that another CTA still has to read), and
 // one cluster barrier per slice orders the deliveries before the next update.
 // The launches of the kernels above, three per slice, each with its fixed
-// cost, were the time of a controller's call: 213 us for ten slices of 1,000
-// neurons, 75 us in one launch.  The ring cells of up to NA_LAGS lags are
-// read ahead of the recurrence, whose lags would else wait for one L2 round
-// trip each.
+// cost, were the time of a controller's call.  The ring cells of up to NA_LAGS
+// lags are read ahead of the recurrence, whose lags would else wait for one L2
+// round trip each.
+// Why 16 CTAs: the adds of a busy network are issued by the cluster's SMs
+// alone, where the per-slice launches have 64 CTAs on as many SMs.  Ten slices
+// by 8 CTAs, by 16, by launches [us]: 1,000 neurons x 100 inputs at 68 Hz 80,
+// 75, 237; 4,000 x 600 at 116 Hz 470, 292, 399; 8,192 x 600 at 188 Hz 1,255,
+// 753, 963; 8,192 x 2,000 at 300 Hz 5,992, 3,419, 5,446.  With 16 the one launch
+// was the faster form at every size from 100 neurons and every rate up to what
+// refractoriness allows (25 to 2,000 inputs); with 8 it was the slower one above
+// some 1e6 edges at 70 to 200 Hz.
 // ---------------------------------------------------------------------
-constexpr int NA_CL_CTAS = 8;   // (the portable cluster size)
+constexpr int NA_CL_CTAS = 16;  // (above the portable 8: a device that cannot place it takes the launches per slice)
+constexpr int NA_CL_TPB = 512;  // threads per CTA: the neurons, and warps to share the deliveries
 constexpr int NA_LAGS = 8;
-constexpr int NA_LIST = 1024 * NA_LAGS;  // a CTA's spikes held at a time
+constexpr int NA_LIST = NA_CL_TPB * NA_LAGS;  // a CTA's spikes held at a time
 
 __device__ __forceinline__ void
 na_cluster_sync()
@@ -219,7 +227,7 @@ na_deliver_spike( const NaNet& d, int src, int slot0, unsigned long long& skippe
   }
 }
 
-__global__ void __launch_bounds__( 1024 )
+__global__ void __launch_bounds__( NA_CL_TPB )
 k_na_run( NaNet d, int per, long long start, long long n_steps, int fresh )
 {
   __shared__ uint32_t s_list[ NA_LIST ];  // local neuron, lag of the chunk << 16
@@ -424,6 +432,7 @@ k_na_finish( NaNet d )
 std::mutex g_na_mutex;
 void* g_na_addr[ NA_MAX_DEVICES ] = {};
 NaRun g_na_run[ NA_MAX_DEVICES ];
+int g_na_cluster[ NA_MAX_DEVICES ] = {};  // 0: not asked yet, 1: the device places k_na_run's cluster, -1: not
 
 }  // namespace
 
@@ -531,21 +540,29 @@ ng_simulate_noalloc( const ng_noalloc_net* net, int64_t n_steps, void* cuda_stre
   // until this call has been enqueued, no later call may continue its run
   run.valid = false;
   cudaError_t ce;
-  if ( net->n <= NA_CL_CTAS * 1024 )
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3( NA_CL_CTAS );
+  lc.blockDim = dim3( NA_CL_TPB );
+  lc.stream = st;
+  cudaLaunchAttribute at[ 1 ];
+  at[ 0 ].id = cudaLaunchAttributeClusterDimension;
+  at[ 0 ].val.clusterDim.x = NA_CL_CTAS;
+  at[ 0 ].val.clusterDim.y = 1;
+  at[ 0 ].val.clusterDim.z = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  if ( !g_na_cluster[ dev ] )
   {
-    // CTAs of 512 threads at least: their warps share the deliveries
+    // once per device: can it place the cluster?
+    int clusters = 0;
+    const bool ok = cudaFuncSetAttribute( k_na_run, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 ) == cudaSuccess
+      && cudaOccupancyMaxActiveClusters( &clusters, k_na_run, &lc ) == cudaSuccess && clusters > 0;
+    cudaGetLastError();  // (a refusal leaves no error behind)
+    g_na_cluster[ dev ] = ok ? 1 : -1;
+  }
+  if ( net->n <= NA_CL_CTAS * NA_CL_TPB && g_na_cluster[ dev ] > 0 )
+  {
     const int per = ( int ) ( ( net->n + NA_CL_CTAS - 1 ) / NA_CL_CTAS );
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3( NA_CL_CTAS );
-    lc.blockDim = dim3( ( unsigned ) std::max( 512, ( per + 31 ) / 32 * 32 ) );
-    lc.stream = st;
-    cudaLaunchAttribute at[ 1 ];
-    at[ 0 ].id = cudaLaunchAttributeClusterDimension;
-    at[ 0 ].val.clusterDim.x = NA_CL_CTAS;
-    at[ 0 ].val.clusterDim.y = 1;
-    at[ 0 ].val.clusterDim.z = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
     if ( cudaLaunchKernelEx( &lc, k_na_run, d, per, ( long long ) net->start_step, ( long long ) n_steps,
            net->continue_run ? 0 : 1 )
       != cudaSuccess )
