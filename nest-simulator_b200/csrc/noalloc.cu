@@ -177,9 +177,13 @@ k_na_deliver( NaNet d )
 // 753, 963; 8,192 x 2,000 at 300 Hz 5,992, 3,419, 5,446.  With 16 the one launch
 // was the faster form at every size from 100 neurons and every rate up to what
 // refractoriness allows (25 to 2,000 inputs); with 8 it was the slower one above
-// some 1e6 edges at 70 to 200 Hz.
+// some 1e6 edges at 70 to 200 Hz.  Networks of up to NA_CL_SMALL neurons have so
+// few adds that the dearer barrier of 16 CTAs is what remains (257 neurons, 285
+// steps: 127.0 us with 8, 128.5 with 16; 319, 164 steps: 75.8 and 77.5; 587 and
+// more: 16 no slower).
 // ---------------------------------------------------------------------
 constexpr int NA_CL_CTAS = 16;  // (above the portable 8: a device that cannot place it takes the launches per slice)
+constexpr int NA_CL_SMALL = 512;
 constexpr int NA_CL_TPB = 512;  // threads per CTA: the neurons, and warps to share the deliveries
 constexpr int NA_LAGS = 8;
 constexpr int NA_LIST = NA_CL_TPB * NA_LAGS;  // a CTA's spikes held at a time
@@ -540,6 +544,7 @@ ng_simulate_noalloc( const ng_noalloc_net* net, int64_t n_steps, void* cuda_stre
   // until this call has been enqueued, no later call may continue its run
   run.valid = false;
   cudaError_t ce;
+  const int ctas = net->n <= NA_CL_SMALL ? NA_CL_CTAS / 2 : NA_CL_CTAS;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3( NA_CL_CTAS );
   lc.blockDim = dim3( NA_CL_TPB );
@@ -562,7 +567,8 @@ ng_simulate_noalloc( const ng_noalloc_net* net, int64_t n_steps, void* cuda_stre
   }
   if ( net->n <= NA_CL_CTAS * NA_CL_TPB && g_na_cluster[ dev ] > 0 )
   {
-    const int per = ( int ) ( ( net->n + NA_CL_CTAS - 1 ) / NA_CL_CTAS );
+    const int per = ( int ) ( ( net->n + ctas - 1 ) / ctas );
+    lc.gridDim.x = at[ 0 ].val.clusterDim.x = ( unsigned ) ctas;
     if ( cudaLaunchKernelEx( &lc, k_na_run, d, per, ( long long ) net->start_step, ( long long ) n_steps,
            net->continue_run ? 0 : 1 )
       != cudaSuccess )
