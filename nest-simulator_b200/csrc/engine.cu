@@ -1201,10 +1201,14 @@ struct ng_engine
     else
     {
       const unsigned grid = ( unsigned ) std::max< int64_t >( 1, ( db.n + P2_NB - 1 ) / P2_NB );
-      if ( v == 2 )
-        k_update_iaf2< Real, FIX, MODEL, 256, 32 ><<< grid, 256, 0, stream >>>( d, db, from_, to_, sched );
+      if ( plastic_on && v == 2 )
+        k_update_iaf2< Real, FIX, MODEL, 256, 32, true ><<< grid, 256, 0, stream >>>( d, db, from_, to_, sched );
+      else if ( plastic_on )
+        k_update_iaf2< Real, FIX, MODEL, 128, 16, true ><<< grid, 128, 0, stream >>>( d, db, from_, to_, sched );
+      else if ( v == 2 )
+        k_update_iaf2< Real, FIX, MODEL, 256, 32, false ><<< grid, 256, 0, stream >>>( d, db, from_, to_, sched );
       else
-        k_update_iaf2< Real, FIX, MODEL, 128, 16 ><<< grid, 128, 0, stream >>>( d, db, from_, to_, sched );
+        k_update_iaf2< Real, FIX, MODEL, 128, 16, false ><<< grid, 128, 0, stream >>>( d, db, from_, to_, sched );
     }
   }
 

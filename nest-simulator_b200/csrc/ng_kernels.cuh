@@ -1019,8 +1019,11 @@ constexpr int P2_NB = 32;  // neurons per CTA
 // TPB threads per CTA, CH lags per chunk (the autotuner picks between
 // 256 threads with chunks of 32 lags and 128 threads with chunks of 16:
 // the same phase-1 items per thread, half the CTA -- more CTAs resident
-// per SM where the registers of the 256-thread form allow only one)
-template < typename Real, bool FIX, int MODEL, int TPB, int CH >
+// per SM where the registers of the 256-thread form allow only one).
+// LAGS: each neuron's lag bits of the slice are kept in gmask, for the plastic
+// connections (a form of its own: in the others the writes cost registers, up
+// to twice the spills, and 0.27 us of 16 us per slice of 568 neurons)
+template < typename Real, bool FIX, int MODEL, int TPB, int CH, bool LAGS >
 __global__ void __launch_bounds__( TPB )
 k_update_iaf2( Net d, Block b, int from, int to, int sched )
 {
@@ -1255,9 +1258,9 @@ k_update_iaf2( Net d, Block b, int from, int to, int sched )
         if ( ++slot == d.L )
           slot = 0;
       }
-      if ( d.gmask && act )
+      if ( LAGS && act )
       {
-        // lag bits of the slice for the plastic connections (min_delay <= 32)
+        // lag bits of the slice (min_delay <= 32)
         if ( cb == 0 )
           d.gmask[ i ] = smask;
         else
