@@ -456,7 +456,7 @@ def measure(args, nest, KERNEL, form, precision, copies, seed, local, dev, pg, e
 
     tuned = eng.tuned()
     upd_name = tuned.get("update_kernel", "k_update_iaf")
-    if upd_name == "k_run_slices":
+    if upd_name in ("k_run_slices", "k_run_slices_mg", "k_run_owned"):
         # one launch runs node update and delivery of many slices: its bytes are
         # both phases' for every slice it covers
         sl = (p1["slices"] - p0["slices"]) / max(1, n_upd)

@@ -292,6 +292,35 @@ int ng_set_tuning( ng_engine* eng, int32_t mode, int32_t update_variant, int32_t
 /* The configuration in force and the autotuner's trials. */
 int ng_get_tuning( ng_engine* eng, ng_tuning* out );
 
+/* The forms that run full min_delay slices. */
+#define NG_FORM_NONE 0     /* no full slice has run yet */
+#define NG_FORM_KERNELS 1  /* update and delivery kernels per slice */
+#define NG_FORM_SCATTER 2  /* k_run_slices: many slices in one launch, one resident wave */
+#define NG_FORM_SCATTER_MG 3 /* k_run_slices_mg: the same for larger networks */
+#define NG_FORM_OWNED 4    /* k_run_owned: many slices in one launch, each SM owning its targets */
+
+/* Which form ran, and the target-owning kernel's layout for the network as it
+ * is connected now (own_* below it are those of the last layout built). */
+typedef struct
+{
+  int32_t form;           /* of the last full slice: NG_FORM_* */
+  int32_t update_variant; /* the update kernel of NG_FORM_KERNELS, numbered as in ng_tuning */
+  int64_t slices[ 5 ];    /* full slices run so far, by form */
+  int32_t own_state;      /* 0: not built, 1: built, -1: the network does not suit the kernel */
+  int32_t own_cell;       /* ring cells: 0 event counts, 1 fixed point, 2 FP64 */
+  int32_t own_window;     /* ring slots in shared memory ... */
+  int32_t own_slots;      /* ... of this many (longer delays go through the global ring) */
+  int32_t own_held;       /* 1: at most one neuron per thread, its state in registers */
+  int32_t own_parts;      /* mutually unconnected parts with SMs of their own */
+  int32_t own_ctas;
+  int32_t own_neurons;    /* most neurons of a CTA */
+  int64_t own_edges;      /* edge copies, padding included ... */
+  int64_t own_far_edges;  /* ... of these, with delays beyond the window */
+  int64_t own_bytes;      /* device memory the layout holds */
+} ng_slice_form;
+
+int ng_get_slice_form( ng_engine* eng, ng_slice_form* out );
+
 /* Engine options: "late_delivery" (1/0: edges of delay >= 2 min_delay
  * delivered on a second stream beside the next slice's update),
  * "late_ctas_per_sm", "aeif_binning" (1/0, default 0: aeif_cond_alpha

@@ -755,6 +755,11 @@ struct ng_engine
   size_t own_smem_bytes = 0;
   OwnNet own_net_d {};
   uint64_t own_seq = 0;      // slices published so far (tags of the exchange buffer)
+  int own_n_parts = 0, own_n_loc = 0;
+  int64_t own_edges = 0, own_far_edges = 0;
+  // full slices run so far, by form, and the last one's form (ng_get_slice_form)
+  int64_t form_slices[ 5 ] = { 0, 0, 0, 0, 0 };
+  int last_form = NG_FORM_NONE;
   // ---- stdp_pl_synapse_hom connections (ng_set_plastic_connections)
   bool plastic_on = false;
   DevBuf pl_row, pl_tgt, pl_dly, pl_w, pl_Kplus, pl_tlast, pl_ninc, pl_tauinv, pl_Kminus, pl_last, pl_hist_t, pl_hist_K,
@@ -1174,17 +1179,35 @@ struct ng_engine
     }
   }
 
+  // the update kernel a block of n neurons runs per slice (or part of one) of
+  // `span` steps: the tuned (or default) kernel; one thread per neuron for 1-2
+  // steps and for engines with the per-target gather or the target-tiled
+  // delivery (the network's mode and spike count are kept there)
+  int
+  kernel_variant( int64_t n, int span ) const
+  {
+    const int v = upd_variant >= 0 && upd_variant != 5 ? upd_variant : engine_default_variant( n );
+    if ( span <= 2 || gather_on || tiled_on )
+      return ( v == 1 || v == 6 ) ? v : 0;
+    return v;
+  }
+
+  // ... of a full slice of the first iaf block
+  int
+  kernels_variant() const
+  {
+    for ( const auto& b : blk )
+      if ( b.model != NG_AEIF_COND_ALPHA )
+        return kernel_variant( b.n, cfg.min_delay );
+    return 4;
+  }
+
   template < typename Real, bool FIX, int MODEL >
   void
   launch_iaf_g( const Net& d, const Block& db, int from_, int to_, int sched )
   {
     const int span = to_ - from_;
-    // the tuned (or default) kernel; one thread per neuron for 1-2 step
-    // slices and for engines with the per-target gather or the target-tiled
-    // delivery (the network's mode and spike count are kept there)
-    int v = upd_variant >= 0 && upd_variant != 5 ? upd_variant : engine_default_variant( db.n );
-    if ( span <= 2 || gather_on || tiled_on )
-      v = ( v == 1 || v == 6 ) ? v : 0;
+    const int v = kernel_variant( db.n, span );
     if ( v <= 1 || v == 6 )
     {
       // CTAs of 4 warps: a large network's grid is resident in one wave
@@ -1570,6 +1593,10 @@ struct ng_engine
     own_cell = cell;
     own_grid = grid;
     own_net = id;
+    own_n_loc = n_loc;
+    own_n_parts = 0;
+    for ( int c = 0; c < grid; c += cta[ ( size_t ) c ].G )
+      ++own_n_parts;
     o.far = W < L ? 1 : 0;
     if ( o.far )
     {
@@ -1588,6 +1615,8 @@ struct ng_engine
     own_seq = 0;
     // near edges, then far ones, in one array each of words and weights
     const size_t edges = 4 * ( size_t ) ( quads + quads_far );
+    own_edges = ( int64_t ) edges;
+    own_far_edges = 4 * quads_far;
     for ( long long& x : ebf )
       x += quads;
     if ( ( rc = upload( own_eb, eb.data(), eb.size() * 8 ) ) || ( rc = upload( own_ebf, ebf.data(), ebf.size() * 8 ) )
@@ -1997,6 +2026,13 @@ struct ng_engine
     return NG_OK;
   }
 
+  void
+  count_form( int form, int64_t k )
+  {
+    last_form = form;
+    form_slices[ form ] += k;
+  }
+
   // enqueue n steps without host synchronisation (except when profiling)
   int
   enqueue_steps( int64_t n )
@@ -2036,6 +2072,7 @@ struct ng_engine
         slices += k;
         n -= st;
         stats.update_launches += 1;
+        count_form( owned > 0 ? NG_FORM_OWNED : pk_multi_group() ? NG_FORM_SCATTER_MG : NG_FORM_SCATTER, k );
         continue;
       }
       if ( from == 0 && graph_slices > 0 && n >= cfg.min_delay )
@@ -2070,6 +2107,7 @@ struct ng_engine
         n -= st;
         stats.update_launches += ( int64_t ) k * ( int64_t ) blk.size();
         stats.deliver_launches += k;
+        count_form( NG_FORM_KERNELS, k );
         continue;
       }
       const int to_ = ( int ) std::min< int64_t >( from + n, cfg.min_delay );
@@ -2082,6 +2120,7 @@ struct ng_engine
         origin += cfg.min_delay;
         from = 0;
         slices += 1;
+        count_form( NG_FORM_KERNELS, 1 );
       }
       else
       {
@@ -3876,6 +3915,32 @@ ng_get_tuning( ng_engine* e, ng_tuning* out )
     out->cand_group[ k ] = c.group;
     out->cand_us_per_slice[ k ] = e->trial_steps > 0 ? c.us * e->cfg.min_delay / ( double ) e->trial_steps : 0.0;
   }
+  return NG_OK;
+}
+
+int
+ng_get_slice_form( ng_engine* e, ng_slice_form* out )
+{
+  if ( !e || !out )
+    return fail( NG_ERR_ARG, "null argument" );
+  std::memset( out, 0, sizeof( *out ) );
+  out->form = e->last_form;
+  out->update_variant = e->kernels_variant();
+  for ( int k = 0; k < 5; ++k )
+    out->slices[ k ] = e->form_slices[ k ];
+  out->own_state = e->own_state;
+  out->own_cell = e->own_cell;
+  out->own_window = e->own_net_d.W;
+  out->own_slots = e->L;
+  out->own_held = e->own_held ? 1 : 0;
+  out->own_parts = e->own_n_parts;
+  out->own_ctas = e->own_grid;
+  out->own_neurons = e->own_n_loc;
+  out->own_edges = e->own_edges;
+  out->own_far_edges = e->own_far_edges;
+  for ( const DevBuf* b : { &e->own_cta, &e->own_rpb, &e->own_rp, &e->own_eb, &e->own_rpf, &e->own_ebf, &e->own_word,
+          &e->own_weight, &e->own_x } )
+    out->own_bytes += ( int64_t ) b->bytes;
   return NG_OK;
 }
 

@@ -34,7 +34,7 @@ EXPORTED = [
     "ng_set_profiling", "ng_set_stream", "ng_set_graph_slices", "ng_debug_coefficients", "ng_net_add", "ng_net_poll",
     "ng_net_spikes", "ng_net_get_var", "ng_net_get_connections", "ng_net_remove", "ng_net_capacity",
     "ng_simulate_noalloc", "ng_set_tuning", "ng_get_tuning", "ng_set_option", "ng_update",
-    "ng_set_plastic_connections", "ng_get_plastic_weights",
+    "ng_set_plastic_connections", "ng_get_plastic_weights", "ng_get_slice_form",
 ]
 
 
@@ -219,6 +219,7 @@ def load():
         "ng_get_spikes": ([P, P, P, i64, P], ctypes.c_int),
         "ng_trace_count": ([P, P, P], ctypes.c_int),
         "ng_get_trace": ([P, P, i64, P], ctypes.c_int),
+        "ng_get_slice_form": ([P, P], ctypes.c_int),
         "ng_get_stats": ([P, P], ctypes.c_int),
         "ng_set_profiling": ([P, i32], ctypes.c_int),
         "ng_set_stream": ([P, P], ctypes.c_int),
@@ -279,6 +280,25 @@ class NGTuning(ctypes.Structure):
     ]
 
 
+class NGSliceForm(ctypes.Structure):
+    _fields_ = [
+        ("form", ctypes.c_int32),
+        ("update_variant", ctypes.c_int32),
+        ("slices", ctypes.c_int64 * 5),
+        ("own_state", ctypes.c_int32),
+        ("own_cell", ctypes.c_int32),
+        ("own_window", ctypes.c_int32),
+        ("own_slots", ctypes.c_int32),
+        ("own_held", ctypes.c_int32),
+        ("own_parts", ctypes.c_int32),
+        ("own_ctas", ctypes.c_int32),
+        ("own_neurons", ctypes.c_int32),
+        ("own_edges", ctypes.c_int64),
+        ("own_far_edges", ctypes.c_int64),
+        ("own_bytes", ctypes.c_int64),
+    ]
+
+
 UPDATE_VARIANTS = {0: "k_update_iaf (one thread per neuron, 4 lags of inputs at a time)",
                    1: "k_update_iaf (one thread per neuron, 8 lags of inputs at a time)",
                    2: "k_update_iaf2 (two-phase, 32 neurons per 256-thread CTA)",
@@ -288,7 +308,8 @@ UPDATE_VARIANTS = {0: "k_update_iaf (one thread per neuron, 4 lags of inputs at 
                       "each SM owning its targets; networks it does not suit: k_run_slices, k_run_slices_mg)",
                    6: "k_update_iaf (one thread per neuron, 2 lags of inputs at a time)"}
 UPDATE_KERNELS = {0: "k_update_iaf", 1: "k_update_iaf", 2: "k_update_iaf2", 3: "k_update_iaf2", 4: "k_update_aeif",
-                  5: "k_run_slices", 6: "k_update_iaf"}
+                  5: "k_run_owned or k_run_slices", 6: "k_update_iaf"}
+FORMS = ("none", "kernels", "k_run_slices", "k_run_slices_mg", "k_run_owned")
 
 
 def tuning_dict(t):
@@ -463,10 +484,24 @@ class Engine:
 
     def tuned(self):
         """The launch configuration the engine runs with (and, once the
-        autotuner has run, what it measured)."""
+        autotuner has run, what it measured).  update_kernel names the kernel
+        that ran the last full slice."""
         t = NGTuning()
         check(self.L.ng_get_tuning(self.handle, ctypes.byref(t)))
-        return tuning_dict(t)
+        d, f = tuning_dict(t), self.slice_form()
+        if f["form"] != "none":
+            d["update_kernel"] = UPDATE_KERNELS[f["update_variant"]] if f["form"] == "kernels" else f["form"]
+        return d
+
+    def slice_form(self):
+        """Which form ran the engine's full slices (and how many each), and
+        the target-owning kernel's layout."""
+        f = NGSliceForm()
+        check(self.L.ng_get_slice_form(self.handle, ctypes.byref(f)))
+        d = {name: getattr(f, name) for name, _ in NGSliceForm._fields_}
+        d["form"] = FORMS[f.form]
+        d["slices"] = dict(zip(FORMS[1:], list(f.slices)[1:]))
+        return d
 
     def set_tuning(self, mode=1, update_variant=-1, deliver_ctas_per_sm=-1, deliver_chunks_per_warp=-1):
         """mode 1: autotune (process cache first), 2: autotune ignoring the

@@ -1,0 +1,90 @@
+"""That the networks of test_gpu_owned.py run in the target-owning kernel, in
+the layouts they are there for: an engine that quietly took another form would
+pass the comparison of results."""
+
+import numpy as np
+import pytest
+
+import test_gpu_owned as owned
+from nestgpu import _abi
+
+pytestmark = pytest.mark.gpu
+
+COUNT, FIXED, F64 = 0, 1, 2
+# (cell, held: at most one neuron per thread, window shorter than the longest delay, parts), case by case.
+# None: the kernel does not take the network (the window would be below min_delay + 16 slots).
+WANT = [(COUNT, 1, False, 1), (COUNT, 1, False, 1), (F64, 1, False, 1), (FIXED, 1, False, 1), (F64, 1, False, 1),
+        (COUNT, 1, False, 1), (F64, 1, False, 1), (COUNT, 1, False, 1), (COUNT, 1, False, 5), (FIXED, 1, False, 1),
+        (FIXED, 0, True, 1), None]
+# layouts that no case there has: two neurons per thread with FP64 cells and with counts, counts with far segments
+MORE = [
+    ((_abi.NG_FP64, owned.DELTA, 80021, 1, 12, 4, 40, False, True, False, (160,)), (F64, 0, True, 1)),
+    ((_abi.NG_FP64, owned.EXP, 76801, 1, 12, 1, 20, False, False, False, (160,)), (F64, 0, True, 1)),
+    ((_abi.NG_FP64, owned.EXP, 80021, 1, 12, 2, 70, True, True, False, (160,)), (COUNT, 0, True, 1)),
+    ((_abi.NG_FP32, owned.EXP, 80021, 1, 12, 2, 20, True, False, True, (160,)), (COUNT, 0, False, 1)),
+    ((_abi.NG_FP64, owned.EXP, 40009, 1, 20, 3, 190, True, False, False, (450,)), (COUNT, 1, True, 1)),
+]
+
+
+def _forms(monkeypatch):
+    """Every engine closed from here on leaves its slice form in the list."""
+    seen, close = [], _abi.Engine.close
+
+    def closing(self):
+        if self.handle:
+            seen.append((self.slice_form(), self.tuned()))
+        close(self)
+
+    monkeypatch.setattr(_abi.Engine, "close", closing)
+    return seen
+
+
+def _check(case, want, f, tuned, out):
+    md, hot, calls = case[5], case[8], case[-1]
+    total = sum(calls) // md
+    assert sum(f["slices"].values()) == total
+    if want is None:
+        assert f["own_state"] == -1 and f["slices"]["k_run_owned"] == 0
+        return
+    # all but what a call starts or ends with in the middle of a slice, and calls of a few slices
+    assert f["slices"]["k_run_owned"] >= total - 8 * len(calls) and f["slices"]["k_run_owned"] > 0
+    cell, held, far, parts = want
+    assert f["own_state"] == 1 and f["own_cell"] == cell and f["own_held"] == held and f["own_parts"] == parts
+    assert (f["own_window"] < f["own_slots"]) == far == (f["own_far_edges"] > 0)
+    assert f["own_ctas"] >= parts and f["own_ctas"] * f["own_neurons"] >= case[2] * case[3]
+    if sum(calls) % md == 0 and calls[-1] >= 16 * md:
+        assert f["form"] == tuned["update_kernel"] == "k_run_owned"
+    if hot:
+        # more spikes in a slice than the kernel's list holds (4,096)
+        assert np.bincount((out[1] - 1) // md).max() > 4096
+
+
+@pytest.mark.parametrize("k", range(len(owned.CASES)))
+def test_layout_of(monkeypatch, k):
+    seen = _forms(monkeypatch)
+    out = owned._run(5, *owned.CASES[k])[0]
+    _check(owned.CASES[k], WANT[k], *seen[0], out)
+
+
+@pytest.mark.parametrize("case,want", MORE)
+def test_more_layouts(monkeypatch, case, want):
+    seen = _forms(monkeypatch)
+    ref, st0 = owned._run(0, *case)[:2]
+    got, st1 = owned._run(5, *case)[:2]
+    _check(case, want, *seen[1], got)
+    assert len(ref[0]) > 20 and st0 == st1
+    for a, b in zip(got, ref):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_what_ran_is_named(monkeypatch):
+    seen = _forms(monkeypatch)
+    case = list(owned.CASES[1])
+    case[-1] = (300,)
+    owned._run(0, *case)
+    owned._run(5, *case)
+    assert [(f["form"], t["update_kernel"]) for f, t in seen] == [("kernels", "k_update_iaf"),
+                                                                  ("k_run_owned", "k_run_owned")]
+    assert seen[0][0]["own_state"] == 0 and seen[0][0]["own_bytes"] == 0
+    # at least the two bytes of an edge word
+    assert seen[1][0]["own_bytes"] > 2 * seen[1][0]["own_edges"] > 0
