@@ -1387,12 +1387,11 @@ struct ng_engine
 
   // Contiguous, mutually unconnected parts of the network (the copies of a
   // batch): each gets SMs of its own, so a spike is exchanged and looked up
-  // among its own part's only.  More parts than SMs: one part.
+  // among its own part's only.
   int
   own_parts( int64_t a, int64_t n, std::vector< OwnCta >& cta, int* nl )
   {
-    std::vector< std::pair< int, int > > part;  // [first, end) of each part
-    std::vector< int64_t > load;
+    std::vector< OwnPart > part;
     if ( !serving )
     {
       void* d_span = nullptr;
@@ -1412,35 +1411,80 @@ struct ng_engine
       CU( ce );
       for ( int64_t s = 0; s < n; ++s )
       {
-        int lo = std::min( ( int ) s, span[ ( size_t ) s ].x ), hi = std::max( ( int ) s, span[ ( size_t ) s ].y ) + 1;
-        int64_t e = deg[ ( size_t ) s ] + 1;
-        while ( !part.empty() && part.back().second > lo )
+        OwnPart p { std::min( ( int ) s, span[ ( size_t ) s ].x ), std::max( ( int ) s, span[ ( size_t ) s ].y ) + 1,
+          ( int64_t ) deg[ ( size_t ) s ] + OWN_NEURON_EDGES };
+        while ( !part.empty() && part.back().end > p.first )
         {
-          lo = std::min( lo, part.back().first );
-          hi = std::max( hi, part.back().second );
-          e += load.back();
+          p.join( part.back() );
           part.pop_back();
-          load.pop_back();
         }
-        part.emplace_back( lo, hi );
-        load.push_back( e );
+        part.push_back( p );
       }
+      own_join_parts( part );
     }
-    if ( part.empty() || ( int64_t ) part.size() > sms )
+    if ( part.size() > 1 )
     {
-      part.assign( 1, { ( int ) a, ( int ) ( a + n ) } );
-      load.assign( 1, 1 );
+      own_share_sms( part, cta, nl );
+      if ( *nl <= 2 * OW_TPB )
+        return NG_OK;
     }
-    // SMs per part: one each, then one at a time to the part with the most
-    // edges per SM, down to OWN_MIN_NEURONS neurons per SM
+    // one network (or parts whose neurons would not fit the SMs that their load gives them)
+    part.assign( 1, OwnPart { ( int ) a, ( int ) ( a + n ), 1 } );
+    own_share_sms( part, cta, nl );
+    return NG_OK;
+  }
+
+  struct OwnPart
+  {
+    int first, end;
+    int64_t load;
+    void
+    join( const OwnPart& o )
+    {
+      first = std::min( first, o.first );
+      end = std::max( end, o.end );
+      load += o.load;
+    }
+  };
+
+  // Parts of less than one SM's share of the load (neurons without any
+  // connection, small networks beside a large one) are joined with their
+  // neighbours -- joined parts are one network whose halves happen not to be
+  // connected -- so that no SM is given to a few neurons.
+  void
+  own_join_parts( std::vector< OwnPart >& part ) const
+  {
+    int64_t total = 0;
+    for ( const OwnPart& p : part )
+      total += p.load;
+    std::vector< OwnPart > out;
+    for ( const OwnPart& p : part )
+      if ( !out.empty() && out.back().load * sms < total )
+        out.back().join( p );
+      else
+        out.push_back( p );
+    if ( out.size() > 1 && out.back().load * sms < total )
+    {
+      const OwnPart last = out.back();
+      out.pop_back();
+      out.back().join( last );
+    }
+    part.swap( out );
+  }
+
+  // SMs per part: one each, then one at a time to the part with the largest
+  // load per SM, down to OWN_MIN_NEURONS neurons per SM
+  void
+  own_share_sms( const std::vector< OwnPart >& part, std::vector< OwnCta >& cta, int* nl ) const
+  {
     const size_t K = part.size();
     std::vector< int > G( K, 1 );
     for ( int left = sms - ( int ) K; left > 0; --left )
     {
       size_t best = K;
       for ( size_t k = 0; k < K; ++k )
-        if ( ( int64_t ) G[ k ] * OWN_MIN_NEURONS < part[ k ].second - part[ k ].first
-          && ( best == K || load[ k ] * G[ best ] > load[ best ] * G[ k ] ) )
+        if ( ( int64_t ) G[ k ] * OWN_MIN_NEURONS < part[ k ].end - part[ k ].first
+          && ( best == K || part[ k ].load * G[ best ] > part[ best ].load * G[ k ] ) )
           best = k;
       if ( best == K )
         break;
@@ -1450,16 +1494,19 @@ struct ng_engine
     *nl = 0;
     for ( size_t k = 0; k < K; ++k )
     {
-      const int pn = part[ k ].second - part[ k ].first, c0 = ( int ) cta.size();
+      const int pn = part[ k ].end - part[ k ].first, c0 = ( int ) cta.size();
       *nl = std::max( *nl, ( pn + G[ k ] - 1 ) / G[ k ] );
       for ( int g = 0; g < G[ k ]; ++g )
         cta.push_back( OwnCta { part[ k ].first, pn, c0, G[ k ] } );
     }
-    return NG_OK;
   }
   // fewest neurons per SM: below it a network's spikes come from more SMs than
   // they have work for (each polls every other one's)
   static constexpr int OWN_MIN_NEURONS = 16;
+  // a neuron's update in edges, for the parts' loads: some 10 cycles of its SM
+  // per 15-step slice (38 per one-step slice), an edge 0.005 to 0.02 at the
+  // rates the benchmark networks fire at
+  static constexpr int64_t OWN_NEURON_EDGES = 1000;
 
   template < typename T >
   int

@@ -88,3 +88,51 @@ def test_what_ran_is_named(monkeypatch):
     assert seen[0][0]["own_state"] == 0 and seen[0][0]["own_bytes"] == 0
     # at least the two bytes of an edge word
     assert seen[1][0]["own_bytes"] > 2 * seen[1][0]["own_edges"] > 0
+
+
+# neurons, connected networks among them (first, size); the other neurons have no connections
+@pytest.mark.parametrize("n,nets", [
+    (4101, [(0, 4001)]),                            # unconnected neurons behind a network
+    (4101, [(100, 4001)]),                          # ... before it
+    (4130, [(0, 2000), (2100, 2000)]),              # ... and between two
+    (6200, [(31 * k, 31) for k in range(200)]),     # more networks than SMs
+    (5000, [(0, 4950), (4960, 9)]),                 # a network too small for an SM of its own
+])
+def test_parts(n, nets):
+    md = 15
+
+    def run(variant):
+        rng = np.random.default_rng(n)
+        deg = np.zeros(n, dtype=np.int64)
+        for first, size in nets:
+            deg[first:first + size] = rng.integers(10, 40, size)
+        row = np.concatenate([[0], np.cumsum(deg)])
+        src = np.repeat(np.arange(n), deg)
+        tgt = np.zeros(len(src), dtype=np.int32)
+        for first, size in nets:
+            at = (src >= first) & (src < first + size)
+            tgt[at] = rng.integers(first, first + size, at.sum())
+        eng = _abi.Engine([(_abi.NG_IAF_PSC_EXP, n)], 0.1, md, md)
+        eng.set_tuning(0, variant, -1, -1)
+        eng.set_var(0, "V_m_rel", rng.uniform(0.0, 14.5, n))
+        eng.set_connections(row, tgt, np.where(src % 5 < 4, 60.0, -240.0), np.full(len(src), md, dtype=np.int32))
+        eng.set_recording(np.ones(n, dtype=np.uint8))
+        eng.set_poisson(np.full(n, 11000.0), np.full(n, 48.0), np.full(n, md, dtype=np.int32), 0, 10**9, 3)
+        eng.simulate(600)
+        s, t = eng.spikes()
+        o = np.lexsort((s, t))
+        out = [s[o], t[o]] + [eng.get_var(0, v) for v in ("V_m_rel", "I_syn_ex", "I_syn_in")]
+        f = eng.slice_form()
+        eng.close()
+        return out, f
+
+    ref, got = run(0), run(5)
+    assert len(ref[0][0]) > 20
+    for a, b in zip(ref[0], got[0]):
+        np.testing.assert_array_equal(a, b)
+    f = got[1]
+    assert f["slices"]["k_run_owned"] == 40
+    assert f["own_parts"] <= f["own_ctas"]
+    # no SM has much more than its share of the neurons
+    assert f["own_neurons"] <= 2 * -(-n // f["own_ctas"])
+    assert f["own_ctas"] >= 100
