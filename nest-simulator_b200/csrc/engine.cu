@@ -1508,6 +1508,32 @@ struct ng_engine
   // rates the benchmark networks fire at
   static constexpr int64_t OWN_NEURON_EDGES = 1000;
 
+  // A window of W slots, shorter than the longest delay: does the kernel still
+  // beat the network's next best form?  Every input of a slice then has to look
+  // at the global ring too, which only slices of one step can read ahead.
+  // Delays up to a little (three times) beyond the window, all sizes from
+  // 12,500 to 100,000 neurons, against the faster of the scatter and graph
+  // forms [us per slice]: min_delay 1 40,000 neurons 9.1 (9.7) against 14.0
+  // (15.2), 100,000 14.8 (15.6) against 23.8 (25.4); 2 40,000 14.6 (16.9) against
+  // 15.2 (16.5), 100,000 with counts 23.6 (28.5) against 27.6 (29.5); 5 24.0
+  // (31.4) against 18.5 (21.5); 15 55.3 (79.1) against 27.7 (34.8).  How many edges
+  // lie beyond the window matters less than that any do: the refusal is by
+  // min_delay.  FP64 cells against the one-wave scatter form lose at 1 step
+  // too (12,500 neurons 8.4 against 7.6).  A serving engine has the graph form
+  // only (40,000 neurons, 2 steps: 23.1; 76,000, 5 steps: 41.1 against 30.2).
+  bool
+  own_far_pays( int W, int cell, bool held )
+  {
+    const int md = cfg.min_delay;
+    if ( W < md + 16 )  // (the smallest windows measured: 18 slots)
+      return false;
+    if ( serving )
+      return md <= 2;
+    if ( md == 1 )
+      return !( cell == OW_F64 && persistent_ok() && !pk_multi_group() );
+    return md == 2 && cell == OW_COUNT && !held;
+  }
+
   template < typename T >
   int
   own_build_t( int64_t a, int64_t n, int id )
@@ -1627,9 +1653,7 @@ struct ng_engine
     if ( fixed >= room )
       return NG_ERR_CAPACITY;
     const int W = ( int ) std::min< size_t >( ( size_t ) L, ( room - fixed ) / ( ( size_t ) nl * own_cell_bytes( cell, two ) ) );
-    // a window below min_delay + 16 slots would send most arrivals through the
-    // global ring, the scatter form's path
-    if ( W < L && W < md + 16 )
+    if ( W < L && !own_far_pays( W, cell, held ) )
       return NG_ERR_CAPACITY;
     while ( kc < std::min( md, 32 ) && own_smem( cell, two, held, nl, W, md, rsz_i, kc + 1, 0 ).total <= room )
       ++kc;

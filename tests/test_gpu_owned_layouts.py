@@ -12,17 +12,24 @@ pytestmark = pytest.mark.gpu
 
 COUNT, FIXED, F64 = 0, 1, 2
 # (cell, held: at most one neuron per thread, window shorter than the longest delay, parts), case by case.
-# None: the kernel does not take the network (the window would be below min_delay + 16 slots).
+# None: the kernel does not take the network (delays beyond the window at more than one step per slice).
 WANT = [(COUNT, 1, False, 1), (COUNT, 1, False, 1), (F64, 1, False, 1), (FIXED, 1, False, 1), (F64, 1, False, 1),
         (COUNT, 1, False, 1), (F64, 1, False, 1), (COUNT, 1, False, 1), (COUNT, 1, False, 5), (FIXED, 1, False, 1),
         (FIXED, 0, True, 1), None]
 # layouts that no case there has: two neurons per thread with FP64 cells and with counts, counts with far segments
 MORE = [
-    ((_abi.NG_FP64, owned.DELTA, 80021, 1, 12, 4, 40, False, True, False, (160,)), (F64, 0, True, 1)),
+    ((_abi.NG_FP64, owned.DELTA, 80021, 1, 12, 1, 44, False, True, False, (160,)), (F64, 0, True, 1)),
     ((_abi.NG_FP64, owned.EXP, 76801, 1, 12, 1, 20, False, False, False, (160,)), (F64, 0, True, 1)),
     ((_abi.NG_FP64, owned.EXP, 80021, 1, 12, 2, 70, True, True, False, (160,)), (COUNT, 0, True, 1)),
     ((_abi.NG_FP32, owned.EXP, 80021, 1, 12, 2, 20, True, False, True, (160,)), (COUNT, 0, False, 1)),
-    ((_abi.NG_FP64, owned.EXP, 40009, 1, 20, 3, 190, True, False, False, (450,)), (COUNT, 1, True, 1)),
+    ((_abi.NG_FP64, owned.EXP, 40009, 1, 20, 1, 190, True, False, False, (450,)), (COUNT, 1, True, 1)),
+]
+# delays beyond the window in networks whose other forms are faster then
+REFUSED = [
+    (_abi.NG_FP64, owned.DELTA, 80021, 1, 12, 4, 40, False, True, False, (160,)),
+    (_abi.NG_FP64, owned.EXP, 40009, 1, 20, 3, 190, True, False, False, (450,)),
+    (_abi.NG_FP32, owned.EXP, 40009, 1, 20, 2, 70, False, False, False, (300,)),
+    (_abi.NG_FP64, owned.EXP, 12503, 1, 20, 1, 160, False, False, False, (300,)),
 ]
 
 
@@ -75,6 +82,13 @@ def test_more_layouts(monkeypatch, case, want):
     assert len(ref[0]) > 20 and st0 == st1
     for a, b in zip(got, ref):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("case", REFUSED)
+def test_long_delays_keep_the_other_forms(monkeypatch, case):
+    seen = _forms(monkeypatch)
+    owned._run(5, *case)
+    _check(case, None, *seen[0], None)
 
 
 def test_what_ran_is_named(monkeypatch):
