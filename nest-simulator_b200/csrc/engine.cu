@@ -749,7 +749,9 @@ struct ng_engine
   // in-edges, laid out for the network as it is connected now
   int own_state = 0;         // 0: to be built, 1: ready, -1: the network does not qualify
   bool own_drive_ok = true;  // every drive table is a CDF table (no walk from the mode)
-  DevBuf own_cta, own_rpb, own_rp, own_eb, own_rpf, own_ebf, own_word, own_weight, own_x;
+  DevBuf own_tab, own_word, own_tmp;  // tables and exchange regions; edge words and weights; scratch of a build
+  void* own_x = nullptr;              // (in own_tab)
+  size_t own_x_bytes = 0;
   bool own_held = true;
   int own_cell = 0, own_grid = 0, own_net = -1;
   size_t own_smem_bytes = 0;
@@ -832,7 +834,7 @@ struct ng_engine
       &net_spk, &log_sorted, &log_cnt, &log_off, &sc_bound, &seg, &net_t, &row_ue, &row_ls, &ent_late, &pk, &pl_row,
       &pl_tgt, &pl_dly, &pl_w, &pl_Kplus, &pl_tlast, &pl_ninc, &pl_tauinv, &pl_Kminus, &pl_last, &pl_hist_t, &pl_hist_K,
       &pl_hist_n, &pl_hist_lo, &pl_drop_t, &pl_drop_K, &pl_nflush, &pl_in_row, &pl_in_edge, &pl_in_src, &pl_wrun,
-      &pl_tab_fin, &pl_tab_km, &pl_list, &pl_items, &pl_spk, &pl_done, &pl_fitems, &own_cta, &own_rpb, &own_rp, &own_eb, &own_rpf, &own_ebf, &own_word, &own_weight, &own_x };
+      &pl_tab_fin, &pl_tab_km, &pl_list, &pl_items, &pl_spk, &pl_done, &pl_fitems, &own_tab, &own_word, &own_tmp };
     for ( DevBuf* b : bufs )
       cudaFree( b->p );
     if ( host_ctl )
@@ -879,6 +881,27 @@ struct ng_engine
     b.bytes = bytes;
     CU( cudaMemsetAsync( b.p, 0, bytes, stream ) );
     return NG_OK;
+  }
+
+  // room for `bytes`, contents undefined: the buffer as it is where it is large
+  // enough, and not many times too large (no cudaMalloc and no device-wide wait)
+  int
+  reserve( DevBuf& b, size_t bytes )
+  {
+    if ( b.p && b.bytes >= bytes && b.bytes / 4 <= bytes + ( 1u << 20 ) )
+      return NG_OK;
+    release( b );
+    CU( cudaMalloc( &b.p, bytes ) );
+    b.bytes = bytes;
+    return NG_OK;
+  }
+
+  static void
+  release( DevBuf& b )
+  {
+    cudaFree( b.p );
+    b.p = nullptr;
+    b.bytes = 0;
   }
 
   int
@@ -1394,21 +1417,15 @@ struct ng_engine
     std::vector< OwnPart > part;
     if ( !serving )
     {
-      void* d_span = nullptr;
-      CU( cudaMalloc( &d_span, ( size_t ) n * sizeof( int2 ) ) );
+      int2* const d_span = ( int2* ) own_tmp.p;
       std::vector< int2 > span( ( size_t ) n );
       std::vector< int32_t > deg( ( size_t ) n );
       k_own_span<<< ( unsigned ) ( ( n * 32 + 255 ) / 256 ), 256, 0, stream >>>( n, ( const int64_t* ) row_beg.p,
-        ( const int32_t* ) real_deg.p, ( const uint32_t* ) tdc.p, tmask, ( int2* ) d_span );
-      cudaError_t ce = cudaGetLastError();
-      if ( ce == cudaSuccess )
-        ce = cudaMemcpyAsync( span.data(), d_span, ( size_t ) n * sizeof( int2 ), cudaMemcpyDeviceToHost, stream );
-      if ( ce == cudaSuccess )
-        ce = cudaMemcpyAsync( deg.data(), real_deg.p, ( size_t ) n * 4, cudaMemcpyDeviceToHost, stream );
-      if ( ce == cudaSuccess )
-        ce = cudaStreamSynchronize( stream );
-      cudaFree( d_span );
-      CU( ce );
+        ( const int32_t* ) real_deg.p, ( const uint32_t* ) tdc.p, tmask, d_span );
+      CU( cudaGetLastError() );
+      CU( cudaMemcpyAsync( span.data(), d_span, ( size_t ) n * sizeof( int2 ), cudaMemcpyDeviceToHost, stream ) );
+      CU( cudaMemcpyAsync( deg.data(), real_deg.p, ( size_t ) n * 4, cudaMemcpyDeviceToHost, stream ) );
+      CU( cudaStreamSynchronize( stream ) );
       for ( int64_t s = 0; s < n; ++s )
       {
         OwnPart p { std::min( ( int ) s, span[ ( size_t ) s ].x ), std::max( ( int ) s, span[ ( size_t ) s ].y ) + 1,
@@ -1540,7 +1557,9 @@ struct ng_engine
   {
     std::vector< OwnCta > cta;
     int n_loc = 0, rc;
-    if ( ( rc = own_parts( a, n, cta, &n_loc ) ) )
+    // scratch: the parts' spans, then class weight bounds, in-degree maximum, owners' edge totals
+    if ( ( rc = reserve( own_tmp, std::max( ( size_t ) n * sizeof( int2 ), 64 + 2 * ( size_t ) sms * 8 ) ) )
+      || ( rc = own_parts( a, n, cta, &n_loc ) ) )
       return rc;
     if ( n_loc > 2 * OW_TPB )
       return NG_ERR_CAPACITY;
@@ -1555,22 +1574,8 @@ struct ng_engine
       rp_n += cta[ ( size_t ) c ].n + 1;
       n_max = std::max( n_max, cta[ ( size_t ) c ].n );
     }
-    if ( ( rc = upload( own_cta, cta.data(), cta.size() * sizeof( OwnCta ) ) )
-      || ( rc = upload( own_rpb, rpb.data(), rpb.size() * 8 ) ) || ( rc = alloc( own_rp, ( size_t ) rp_n * 4 ) ) )
-      return rc;
-    // scratch: class weight bounds, owners' edge totals, in-degrees per class
-    struct Tmp
-    {
-      void* p = nullptr;
-      ~Tmp() { cudaFree( p ); }
-    } tmp;
-    const size_t head = 64 + ( size_t ) grid * 8;
-    CU( cudaMalloc( &tmp.p, head + ( size_t ) n * 8 ) );
-    unsigned long long* const bounds = ( unsigned long long* ) tmp.p;  // min[2], max[2], in-degree maximum
-    unsigned long long* const total = bounds + 8;
-    unsigned* const indeg = ( unsigned* ) ( ( char* ) tmp.p + head );
-    CU( cudaMemsetAsync( tmp.p, 0, head + ( size_t ) n * 8, stream ) );
-    CU( cudaMemsetAsync( bounds, 0xff, 16, stream ) );
+    unsigned long long* const bounds = ( unsigned long long* ) own_tmp.p;  // min[2], max[2], in-degree maximum
+    unsigned long long* const total = bounds + 8;                         // near, then far, by owner
     OwnBuild q {};
     q.row_beg = ( const int64_t* ) row_beg.p;
     q.real_deg = ( const int32_t* ) real_deg.p;
@@ -1579,50 +1584,24 @@ struct ng_engine
     q.tmask = tmask;
     q.dmask = dmask;
     q.tbits = tbits;
-    q.rp_base = ( const long long* ) own_rpb.p;
-    auto each_part = [ & ]( auto&& f ) {
+    q.split = two ? 0 : 1;
+    auto each_part = [ & ]( int rows, auto&& f ) {
       for ( int c = 0; c < grid; c += cta[ ( size_t ) c ].G )
       {
         q.a = cta[ ( size_t ) c ].a;
         q.n = cta[ ( size_t ) c ].n;
         q.c0 = c;
         q.G = cta[ ( size_t ) c ].G;
-        f( ( unsigned ) std::min( ( q.n + 7 ) / 8, 8 * sms ) );
+        f( ( unsigned ) std::min( ( q.n + rows - 1 ) / rows, 8 * sms ) );
       }
     };
-    std::vector< unsigned long long > host( 8 + ( size_t ) grid );
-    // edges of delay [lo, hi) per owner and source as segment starts; owners' starts and total [quads]
-    auto count = [ & ]( DevBuf& rp, int lo, int hi, bool stats, std::vector< long long >& eb, long long* quads ) -> int {
-      q.rp = ( uint32_t* ) rp.p;
-      q.d_lo = lo;
-      q.d_hi = hi;
-      each_part( [ & ]( unsigned g ) {
-        k_own_count< T ><<< g, 256, 0, stream >>>( q, two ? 0 : 1, stats ? indeg - 2 * a : nullptr, bounds, bounds + 2 );
-      } );
-      if ( stats )
-        k_own_max<<< ( unsigned ) std::min< int64_t >( ( 2 * n + 255 ) / 256, 4 * sms ), 256, 0, stream >>>( 2 * n, indeg,
-          ( unsigned* ) ( bounds + 4 ) );
-      k_own_scan<<< ( unsigned ) grid, 1024, 0, stream >>>( ( const OwnCta* ) own_cta.p, ( const long long* ) own_rpb.p,
-        ( uint32_t* ) rp.p, total );
-      CU( cudaGetLastError() );
-      CU( cudaMemcpyAsync( host.data(), tmp.p, head, cudaMemcpyDeviceToHost, stream ) );
-      CU( cudaStreamSynchronize( stream ) );
-      eb.assign( ( size_t ) grid, 0 );
-      *quads = 0;
-      for ( int c = 0; c < grid; ++c )
-      {
-        eb[ ( size_t ) c ] = *quads;
-        *quads += ( long long ) host[ 8 + ( size_t ) c ];
-      }
-      return NG_OK;
-    };
-    std::vector< long long > eb, ebf;
-    long long quads = 0, quads_far = 0;
-    if ( ( rc = count( own_rp, 0, INT32_MAX, true, eb, &quads ) ) )
-      return rc;
-    // (a cell's 16-bit event count and 16 high bits hold any in-degree up to this)
-    if ( quads == 0 || ( unsigned ) host[ 4 ] > 65000u )
-      return NG_ERR_CAPACITY;
+    std::vector< unsigned long long > host( 8 + 2 * ( size_t ) grid );
+    CU( cudaMemsetAsync( bounds, 0, 64, stream ) );
+    CU( cudaMemsetAsync( bounds, 0xff, 16, stream ) );
+    each_part( 8, [ & ]( unsigned g ) { k_own_bounds< T ><<< g, 256, 0, stream >>>( q, bounds, bounds + 2 ); } );
+    CU( cudaGetLastError() );
+    CU( cudaMemcpyAsync( host.data(), bounds, 64, cudaMemcpyDeviceToHost, stream ) );
+    CU( cudaStreamSynchronize( stream ) );
     // one weight per input class: cells count events
     OwnNet o {};
     bool uniform = true;
@@ -1640,6 +1619,8 @@ struct ng_engine
         std::memcpy( &o.cw[ c ], &u, 8 );
       }
     }
+    if ( host[ 2 ] == 0 && host[ 3 ] == 0 )
+      return NG_ERR_CAPACITY;  // no edges
     const int cell = uniform ? OW_COUNT : fx ? OW_I64 : OW_F64;
     // ring window: all delays where they fit, else the nearest ones, beside the
     // stage of at least 4 lags' inputs (all of the slice's where there is room)
@@ -1669,52 +1650,95 @@ struct ng_engine
     for ( int c = 0; c < grid; c += cta[ ( size_t ) c ].G )
       ++own_n_parts;
     o.far = W < L ? 1 : 0;
-    if ( o.far )
-    {
-      // an edge of delay d arrives d - 1 steps past the next slice's first one at most
-      if ( ( rc = alloc( own_rpf, ( size_t ) rp_n * 4 ) ) || ( rc = count( own_rp, 0, W + 1, false, eb, &quads ) )
-        || ( rc = count( own_rpf, W + 1, INT32_MAX, false, ebf, &quads_far ) ) )
-        return rc;
-    }
     o.x_cap = std::max< long long >( 32, ( long long ) nl * md + 1 );
-    // 2-byte edge words where (delay, local target) fits 15 bits
-    o.w16 = cell == OW_COUNT && ( int64_t ) ( cfg.max_delay + 1 ) * nl < 32768 ? 1 : 0;
-    const size_t wb = cell == OW_I64 ? 8 : o.w16 ? 2 : 4;
-    if ( ( rc = alloc( own_x, 2 * ( size_t ) grid * ( size_t ) o.x_cap * 8 ) )
-      || ( !pk.p && ( rc = alloc( pk, sizeof( PkCtl ) ) ) ) )
+    // tables of the owners: shares, starts, row tables, exchange regions
+    size_t at = 0;
+    auto place = [ &at ]( size_t bytes ) {
+      const size_t p = at;
+      at += ( bytes + 255 ) & ~( size_t ) 255;
+      return p;
+    };
+    const size_t x_bytes = 2 * ( size_t ) grid * ( size_t ) o.x_cap * 8;
+    const size_t p_cta = place( cta.size() * sizeof( OwnCta ) ), p_rpb = place( rpb.size() * 8 ), p_eb = place( rpb.size() * 8 ),
+                 p_ebf = place( rpb.size() * 8 ), p_x = place( x_bytes ), p_rp = place( ( size_t ) rp_n * 4 ),
+                 p_rpf = place( o.far ? ( size_t ) rp_n * 4 : 0 );
+    if ( ( rc = reserve( own_tab, at ) ) || ( !pk.p && ( rc = alloc( pk, sizeof( PkCtl ) ) ) ) )
       return rc;
+    char* const tab = ( char* ) own_tab.p;
+    CU( cudaMemcpyAsync( tab + p_cta, cta.data(), cta.size() * sizeof( OwnCta ), cudaMemcpyHostToDevice, stream ) );
+    CU( cudaMemcpyAsync( tab + p_rpb, rpb.data(), rpb.size() * 8, cudaMemcpyHostToDevice, stream ) );
+    CU( cudaMemsetAsync( tab + p_x, 0, x_bytes, stream ) );
     own_seq = 0;
+    own_x = tab + p_x;
+    own_x_bytes = x_bytes;
+    // edges per owner and source as segment starts: an edge of delay d arrives
+    // d - 1 steps past the next slice's first one at most
+    q.rp_base = ( const long long* ) ( tab + p_rpb );
+    q.rp = ( uint32_t* ) ( tab + p_rp );
+    q.rp_far = o.far ? ( uint32_t* ) ( tab + p_rpf ) : nullptr;
+    q.d_near = o.far ? W : INT32_MAX;
+    each_part( 8, [ & ]( unsigned g ) { k_own_count< T ><<< g, 256, 0, stream >>>( q ); } );
+    k_own_scan<<< dim3( ( unsigned ) grid, o.far ? 2 : 1 ), 1024, 0, stream >>>( ( const OwnCta* ) ( tab + p_cta ), q.rp_base,
+      q.rp, q.rp_far, total );
+    CU( cudaGetLastError() );
+    CU( cudaMemcpyAsync( host.data(), bounds, host.size() * 8, cudaMemcpyDeviceToHost, stream ) );
+    CU( cudaStreamSynchronize( stream ) );
     // near edges, then far ones, in one array each of words and weights
+    std::vector< long long > eb( ( size_t ) grid ), ebf( ( size_t ) grid );
+    long long quads = 0, quads_far = 0, most = 0;
+    for ( int c = 0; c < grid; ++c )
+    {
+      eb[ ( size_t ) c ] = quads;
+      quads += ( long long ) host[ 8 + ( size_t ) c ];
+      most = std::max( most, ( long long ) ( host[ 8 + ( size_t ) c ] + ( o.far ? host[ 8 + ( size_t ) ( grid + c ) ] : 0 ) ) );
+    }
+    for ( int c = 0; c < grid && o.far; ++c )
+    {
+      ebf[ ( size_t ) c ] = quads + quads_far;
+      quads_far += ( long long ) host[ 8 + ( size_t ) ( grid + c ) ];
+    }
     const size_t edges = 4 * ( size_t ) ( quads + quads_far );
     own_edges = ( int64_t ) edges;
     own_far_edges = 4 * quads_far;
-    for ( long long& x : ebf )
-      x += quads;
-    if ( ( rc = upload( own_eb, eb.data(), eb.size() * 8 ) ) || ( rc = upload( own_ebf, ebf.data(), ebf.size() * 8 ) )
-      || ( rc = alloc( own_word, edges * wb ) ) || ( rc = alloc( own_weight, cell == OW_F64 ? edges * 8 : 16 ) ) )
+    // 2-byte edge words where (delay, local target) fits 15 bits
+    o.w16 = cell == OW_COUNT && ( int64_t ) ( cfg.max_delay + 1 ) * nl < 32768 ? 1 : 0;
+    const size_t wb = cell == OW_I64 ? 8 : o.w16 ? 2 : 4, word_bytes = ( edges * wb + 255 ) & ~( size_t ) 255;
+    if ( ( rc = reserve( own_word, word_bytes + ( cell == OW_F64 ? edges * 8 : 0 ) ) ) )
       return rc;
-    k_own_pad<<< ( unsigned ) ( 16 * sms ), 256, 0, stream >>>( o.w16, cell == OW_I64 ? 1 : 0, edges,
-      ( uint32_t ) ( md * nl + nl - 1 ), ( uint32_t* ) own_word.p );
-    for ( int f = 0; f <= o.far; ++f )
+    double* const weight = ( double* ) ( ( char* ) own_word.p + word_bytes );
+    CU( cudaMemcpyAsync( tab + p_eb, eb.data(), eb.size() * 8, cudaMemcpyHostToDevice, stream ) );
+    CU( cudaMemcpyAsync( tab + p_ebf, ebf.data(), ebf.size() * 8, cudaMemcpyHostToDevice, stream ) );
+    // rows of many edges per segment by one CTA each, others by a warp (the
+    // fill alone: 6,000 edges a row over 148 owners 4.9 ms against 15.6; the
+    // whole build: 3,000 a row 3.6 against 4.8, 1,250 a row 1.5 against 1.3)
+    const bool rows = edges / ( size_t ) n >= 2048;
+    if ( !rows )
     {
-      q.rp = ( uint32_t* ) ( f ? own_rpf.p : own_rp.p );
-      q.d_lo = f ? W + 1 : 0;
-      q.d_hi = o.far && !f ? W + 1 : INT32_MAX;
-      each_part( [ & ]( unsigned g ) {
-        k_own_fill< T ><<< g, 256, 0, stream >>>( q, two ? 0 : 1, cell, o.w16, nl,
-          ( const long long* ) ( f ? own_ebf.p : own_eb.p ), ( uint32_t* ) own_word.p, ( uint2* ) own_word.p,
-          ( double* ) own_weight.p );
-      } );
+      k_own_pad<<< ( unsigned ) ( 16 * sms ), 256, 0, stream >>>( o.w16, cell == OW_I64 ? 1 : 0, edges,
+        ( uint32_t ) ( md * nl + nl - 1 ), ( uint32_t* ) own_word.p );
+      if ( cell == OW_F64 )
+        CU( cudaMemsetAsync( weight, 0, edges * 8, stream ) );
     }
-    CU( cudaGetLastError() );
-    if ( ( rc = max_dynamic_smem( own_kernel( cell, own_held ) ) ) )
+    constexpr int CW = std::is_same< T, double >::value ? OW_F64 : OW_I64;  // cells of several weights
+    if ( rows
+      && ( rc = max_dynamic_smem( cell == OW_COUNT ? ( const void* ) &k_own_fill_rows< T, OW_COUNT >
+                                                   : ( const void* ) &k_own_fill_rows< T, CW > ) ) )
       return rc;
-    int occ = 0, coop = 0;
-    CU( cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, cfg.device ) );
-    CU( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, own_kernel( cell, own_held ), OW_TPB, own_smem_bytes ) );
-    if ( !coop || occ < 1 )
-      return NG_ERR_CAPACITY;
-    CU( cudaStreamSynchronize( stream ) );
+    each_part( rows ? 1 : 8, [ & ]( unsigned g ) {
+      const long long* const near = ( const long long* ) ( tab + p_eb );
+      const long long* const far = ( const long long* ) ( tab + p_ebf );
+      uint32_t* const word = ( uint32_t* ) own_word.p;
+      const uint32_t pad = ( uint32_t ) ( md * nl + nl - 1 );
+      if ( rows && cell == OW_COUNT )
+        k_own_fill_rows< T, OW_COUNT ><<< g, 512, OW_FILL_SMEM, stream >>>( q, o.w16, nl, pad, near, far, word, weight );
+      else if ( rows )
+        k_own_fill_rows< T, CW ><<< g, 512, OW_FILL_SMEM, stream >>>( q, o.w16, nl, pad, near, far, word, weight );
+      else if ( cell == OW_COUNT )
+        k_own_fill< T, OW_COUNT ><<< g, 256, 0, stream >>>( q, o.w16, nl, near, far, word, weight );
+      else
+        k_own_fill< T, CW ><<< g, 256, 0, stream >>>( q, o.w16, nl, near, far, word, weight );
+    } );
+    CU( cudaGetLastError() );
     // lanes per segment, a quad of edges (OW_COUNT: two) each: 1.4 times the mean segment
     double segs = 0;
     for ( const OwnCta& c : cta )
@@ -1723,19 +1747,44 @@ struct ng_engine
     o.gw_log2 = 0;
     while ( o.gw_log2 < 5 && ( double ) ( ( cell == OW_COUNT ? 2 : 1 ) << o.gw_log2 ) < 1.4 * mean )
       ++o.gw_log2;
-    o.cta = ( const OwnCta* ) own_cta.p;
-    o.rp_base = ( const long long* ) own_rpb.p;
-    o.rp = ( const uint32_t* ) own_rp.p;
-    o.e_base = ( const long long* ) own_eb.p;
-    o.rp_far = ( const uint32_t* ) own_rpf.p;
-    o.e_far = ( const long long* ) own_ebf.p;
+    o.cta = ( const OwnCta* ) ( tab + p_cta );
+    o.rp_base = q.rp_base;
+    o.rp = q.rp;
+    o.e_base = ( const long long* ) ( tab + p_eb );
+    o.rp_far = q.rp_far;
+    o.e_far = ( const long long* ) ( tab + p_ebf );
     o.word = ( const uint4* ) own_word.p;
     o.word_w = ( const uint4* ) own_word.p;
-    o.weight = ( const double2* ) own_weight.p;
-    o.xchg = ( unsigned long long* ) own_x.p;
+    o.weight = ( const double2* ) weight;
+    o.xchg = ( unsigned long long* ) own_x;
     o.nl = nl;
     o.W = W;
     o.pk = ( PkCtl* ) pk.p;
+    // a cell's 16-bit event count and 16 high bits hold any in-degree up to
+    // this (an owner of fewer edges in all has no larger one)
+    constexpr unsigned OWN_IN_DEGREE = 65000u;
+    if ( cell != OW_F64 && 4 * most > ( long long ) OWN_IN_DEGREE )
+    {
+      unsigned* const d_most = ( unsigned* ) ( bounds + 4 );
+      unsigned in_degree = 0;
+      if ( cell == OW_COUNT )
+        k_own_indeg< OW_COUNT ><<< ( unsigned ) grid, 1024, 0, stream >>>( o, total, d_most );
+      else
+        k_own_indeg< OW_I64 ><<< ( unsigned ) grid, 1024, 0, stream >>>( o, total, d_most );
+      CU( cudaGetLastError() );
+      CU( cudaMemcpyAsync( &in_degree, d_most, 4, cudaMemcpyDeviceToHost, stream ) );
+      CU( cudaStreamSynchronize( stream ) );
+      if ( in_degree > OWN_IN_DEGREE )
+        return NG_ERR_CAPACITY;
+    }
+    if ( ( rc = max_dynamic_smem( own_kernel( cell, own_held ) ) ) )
+      return rc;
+    int occ = 0, coop = 0;
+    CU( cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, cfg.device ) );
+    CU( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &occ, own_kernel( cell, own_held ), OW_TPB, own_smem_bytes ) );
+    if ( !coop || occ < 1 )
+      return NG_ERR_CAPACITY;
+    CU( cudaStreamSynchronize( stream ) );  // (eb, ebf and the tables are host vectors of this call)
     own_net_d = o;
     return NG_OK;
   }
@@ -1766,7 +1815,7 @@ struct ng_engine
     // tags are 32 bits wide: start over, with a cleared exchange buffer, long before they repeat
     if ( own_seq + ( uint64_t ) k + 2 > 0xffffffffull )
     {
-      CU( cudaMemsetAsync( own_x.p, 0, own_x.bytes, stream ) );
+      CU( cudaMemsetAsync( own_x, 0, own_x_bytes, stream ) );
       own_seq = 0;
     }
     own_net_d.seq0 = ( unsigned ) ( own_seq + 1 );
@@ -4009,8 +4058,7 @@ ng_get_slice_form( ng_engine* e, ng_slice_form* out )
   out->own_neurons = e->own_n_loc;
   out->own_edges = e->own_edges;
   out->own_far_edges = e->own_far_edges;
-  for ( const DevBuf* b : { &e->own_cta, &e->own_rpb, &e->own_rp, &e->own_eb, &e->own_rpf, &e->own_ebf, &e->own_word,
-          &e->own_weight, &e->own_x } )
+  for ( const DevBuf* b : { &e->own_tab, &e->own_word, &e->own_tmp } )
     out->own_bytes += ( int64_t ) b->bytes;
   return NG_OK;
 }

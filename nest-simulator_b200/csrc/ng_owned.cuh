@@ -1376,7 +1376,8 @@ k_own_span( long long n, const int64_t* row_beg, const int32_t* real_deg, const 
 }
 
 // What the builder works on: rows a .. a + n of one network, owned by the
-// CTAs c0 .. c0 + G.
+// CTAs c0 .. c0 + G.  An edge is near (the segments rp) up to a delay of
+// d_near steps, far (rp_far) beyond.
 struct OwnBuild
 {
   int a, n, c0, G;
@@ -1388,13 +1389,12 @@ struct OwnBuild
   int tbits;
   const long long* rp_base;
   uint32_t* rp;
-  int d_lo, d_hi;  // edges of delay [d_lo, d_hi)
+  uint32_t* rp_far;
+  int d_near;
+  int split;  // a weight's class is its sign instead of its channel (iaf_psc_delta has one channel)
 };
 
-// Edges of every (owner, source); in-degrees per channel; the smallest and
-// largest weight of each class (bit patterns of FP64 or int32 weights mapped
-// to unsigned order).  split: a weight's class is its sign instead of its
-// channel (iaf_psc_delta has one channel).
+// FP64 and int32 weights mapped to unsigned order.
 template < typename T >
 __device__ __forceinline__ unsigned long long
 own_order( T w )
@@ -1408,11 +1408,12 @@ own_order( T w )
     return ( unsigned long long ) ( ( long long ) w + ( 1ll << 40 ) );
 }
 
+// The smallest and largest weight of each class, from the weights alone (the
+// channel of a non-zero weight is its sign, set where the edge was packed).
 template < typename T >
 __global__ void __launch_bounds__( 256 )
-k_own_count( OwnBuild q, int split, unsigned* indeg, unsigned long long* wmin, unsigned long long* wmax )
+k_own_bounds( OwnBuild q, unsigned long long* wmin, unsigned long long* wmax )
 {
-  __shared__ unsigned s_h[ 8 ][ OW_MAX_G ];
   __shared__ unsigned long long s_min[ 2 ], s_max[ 2 ];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if ( threadIdx.x < 2 )
@@ -1424,68 +1425,81 @@ k_own_count( OwnBuild q, int split, unsigned* indeg, unsigned long long* wmin, u
   unsigned long long mn[ 2 ] = { ~0ull, ~0ull }, mx[ 2 ] = { 0ull, 0ull };
   for ( long long s = ( long long ) blockIdx.x * 8 + warp; s < q.n; s += ( long long ) gridDim.x * 8 )
   {
-    for ( int k = lane; k < q.G; k += 32 )
-      s_h[ warp ][ k ] = 0u;
-    __syncwarp();
-    const long long r0 = q.row_beg[ q.a + s ];
+    const T* const w = ( const T* ) q.w + q.row_beg[ q.a + s ];
     const int deg = q.real_deg[ q.a + s ];
+#pragma unroll 4
     for ( int j = lane; j < deg; j += 32 )
     {
-      const T w = ( ( const T* ) q.w )[ r0 + j ];
-      if ( w == T( 0 ) )
+      const T x = w[ j ];
+      const unsigned long long u = own_order< T >( x );
+      const bool second = q.split ? x < T( 0 ) : !( x > T( 0 ) );
+      if ( x == T( 0 ) )
         continue;
-      const uint32_t t = q.tdc[ r0 + j ];
-      const int dl = ( int ) ( ( t >> q.tbits ) & q.dmask );
-      if ( dl < q.d_lo || dl >= q.d_hi )
-        continue;
-      const unsigned l = ( t & q.tmask ) - ( unsigned ) q.a;
-      const unsigned cl = split ? ( w < T( 0 ) ? 1u : 0u ) : t >> 31;
-      atomicAdd( &s_h[ warp ][ l % ( unsigned ) q.G ], 1u );
-      if ( !indeg )
-        continue;  // (counts only)
-      atomicAdd( indeg + 2 * ( size_t ) ( q.a + l ) + cl, 1u );
-      const unsigned long long u = own_order< T >( w );
-      mn[ cl ] = min( mn[ cl ], u );
-      mx[ cl ] = max( mx[ cl ], u );
+      // (selections: an array indexed by the class would be in local memory)
+      mn[ 0 ] = second ? mn[ 0 ] : min( mn[ 0 ], u );
+      mx[ 0 ] = second ? mx[ 0 ] : max( mx[ 0 ], u );
+      mn[ 1 ] = second ? min( mn[ 1 ], u ) : mn[ 1 ];
+      mx[ 1 ] = second ? max( mx[ 1 ], u ) : mx[ 1 ];
     }
-    __syncwarp();
-    for ( int k = lane; k < q.G; k += 32 )
-      q.rp[ q.rp_base[ q.c0 + k ] + s ] = s_h[ warp ][ k ];
-    __syncwarp();
   }
 #pragma unroll
   for ( int c = 0; c < 2; ++c )
-  {
     if ( mx[ c ] )
     {
       atomicMin( &s_min[ c ], mn[ c ] );
       atomicMax( &s_max[ c ], mx[ c ] );
     }
-  }
   __syncthreads();
-  if ( indeg && threadIdx.x < 2 && s_max[ threadIdx.x ] )
+  if ( threadIdx.x < 2 && s_max[ threadIdx.x ] )
   {
     atomicMin( wmin + threadIdx.x, s_min[ threadIdx.x ] );
     atomicMax( wmax + threadIdx.x, s_max[ threadIdx.x ] );
   }
 }
 
-__global__ void
-k_own_max( long long n, const unsigned* v, unsigned* out )
+// Near and far edges of every (owner, source), in one pass over the rows.
+template < typename T >
+__global__ void __launch_bounds__( 256 )
+k_own_count( OwnBuild q )
 {
-  unsigned m = 0;
-  for ( long long k = ( long long ) blockIdx.x * blockDim.x + threadIdx.x; k < n; k += ( long long ) gridDim.x * blockDim.x )
-    m = max( m, v[ k ] );
-  m = __reduce_max_sync( FULL, m );
-  if ( ( threadIdx.x & 31 ) == 0 && m )
-    atomicMax( out, m );
+  __shared__ unsigned s_h[ 8 ][ 2 * OW_MAX_G ];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int G2 = q.rp_far ? 2 * q.G : q.G;
+  for ( long long s = ( long long ) blockIdx.x * 8 + warp; s < q.n; s += ( long long ) gridDim.x * 8 )
+  {
+    for ( int k = lane; k < G2; k += 32 )
+      s_h[ warp ][ k ] = 0u;
+    __syncwarp();
+    const long long r0 = q.row_beg[ q.a + s ];
+    const int deg = q.real_deg[ q.a + s ];
+#pragma unroll 4
+    for ( int j = lane; j < deg; j += 32 )
+    {
+      const T w = ( ( const T* ) q.w )[ r0 + j ];
+      const uint32_t t = q.tdc[ r0 + j ];
+      if ( w == T( 0 ) )
+        continue;
+      const int dl = ( int ) ( ( t >> q.tbits ) & q.dmask );
+      const unsigned l = ( t & q.tmask ) - ( unsigned ) q.a;
+      atomicAdd( &s_h[ warp ][ l % ( unsigned ) q.G + ( dl > q.d_near ? q.G : 0 ) ], 1u );
+    }
+    __syncwarp();
+    for ( int k = lane; k < q.G; k += 32 )
+    {
+      q.rp[ q.rp_base[ q.c0 + k ] + s ] = s_h[ warp ][ k ];
+      if ( q.rp_far )
+        q.rp_far[ q.rp_base[ q.c0 + k ] + s ] = s_h[ warp ][ q.G + k ];
+    }
+    __syncwarp();
+  }
 }
 
-// One CTA per owner: its counts become segment starts in quads of edges
-// (entry n: its total).
+// One CTA per owner (and, blockIdx.y, near or far): its counts become segment
+// starts in quads of edges (entry n: its total).
 __global__ void __launch_bounds__( 1024 )
-k_own_scan( const OwnCta* cta, const long long* rp_base, uint32_t* rp, unsigned long long* total )
+k_own_scan( const OwnCta* cta, const long long* rp_base, uint32_t* rp_near, uint32_t* rp_far, unsigned long long* total )
 {
+  uint32_t* const rp = blockIdx.y ? rp_far : rp_near;
   __shared__ unsigned s_w[ 32 ];
   __shared__ unsigned s_carry;
   const int n = cta[ blockIdx.x ].n;
@@ -1522,7 +1536,7 @@ k_own_scan( const OwnCta* cta, const long long* rp_base, uint32_t* rp, unsigned 
   if ( threadIdx.x == 0 )
   {
     p[ n ] = s_carry;
-    total[ blockIdx.x ] = s_carry;
+    total[ blockIdx.y * gridDim.x + blockIdx.x ] = s_carry;
   }
 }
 
@@ -1539,22 +1553,42 @@ k_own_pad( int w16, int pair, size_t n, uint32_t v, uint32_t* word )
       word[ k ] = v;
 }
 
-// Edges into the owners' segments (any order within a segment).
+// An edge's owner segment (near: owner, far: G + owner) and its word.
 template < typename T >
-__global__ void __launch_bounds__( 256 )
-k_own_fill( OwnBuild q, int split, int cell, int w16, int nl, const long long* e_base, uint32_t* word, uint2* word_w,
-  double* weight )
+__device__ __forceinline__ unsigned
+own_place( const OwnBuild& q, uint32_t t, T w, bool by_sign, int nl, uint32_t& x )
 {
-  __shared__ unsigned s_at[ 8 ][ OW_MAX_G ];
-  __shared__ long long s_base[ OW_MAX_G ];
+  const int dl = ( int ) ( ( t >> q.tbits ) & q.dmask );
+  const unsigned l = ( t & q.tmask ) - ( unsigned ) q.a, c = l / ( unsigned ) q.G, own = l - c * ( unsigned ) q.G;
+  const unsigned cl = by_sign ? ( w < T( 0 ) ? 1u : 0u ) : t >> 31;
+  x = ( ( uint32_t ) dl * ( uint32_t ) nl + c ) | ( cl << 31 );
+  return own + ( dl > q.d_near ? q.G : 0 );
+}
+
+__device__ __forceinline__ uint16_t
+own_word16( uint32_t x )
+{
+  return ( uint16_t ) ( ( x & 0x7fffu ) | ( x >> 16 & 0x8000u ) );
+}
+
+// Edges into the owners' segments (any order within a segment), a row per
+// warp: rows of a few edges per segment.
+template < typename T, int CELL >
+__global__ void __launch_bounds__( 256 )
+k_own_fill( OwnBuild q, int w16, int nl, const long long* e_near, const long long* e_far, uint32_t* word, double* weight )
+{
+  __shared__ unsigned s_at[ 8 ][ 2 * OW_MAX_G ];
+  __shared__ long long s_base[ 2 * OW_MAX_G ];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for ( int k = threadIdx.x; k < q.G; k += blockDim.x )
-    s_base[ k ] = 4 * e_base[ q.c0 + k ];
+  const int G2 = q.rp_far ? 2 * q.G : q.G;
+  for ( int k = threadIdx.x; k < G2; k += blockDim.x )
+    s_base[ k ] = 4 * ( k < q.G ? e_near[ q.c0 + k ] : e_far[ q.c0 + k - q.G ] );
   __syncthreads();
   for ( long long s = ( long long ) blockIdx.x * 8 + warp; s < q.n; s += ( long long ) gridDim.x * 8 )
   {
-    for ( int k = lane; k < q.G; k += 32 )
-      s_at[ warp ][ k ] = 4u * q.rp[ q.rp_base[ q.c0 + k ] + s ];
+    for ( int k = lane; k < G2; k += 32 )
+      s_at[ warp ][ k ] = 4u
+        * ( k < q.G ? q.rp[ q.rp_base[ q.c0 + k ] + s ] : q.rp_far[ q.rp_base[ q.c0 + k - q.G ] + s ] );
     __syncwarp();
     const long long r0 = q.row_beg[ q.a + s ];
     const int deg = q.real_deg[ q.a + s ];
@@ -1563,28 +1597,236 @@ k_own_fill( OwnBuild q, int split, int cell, int w16, int nl, const long long* e
       const T w = ( ( const T* ) q.w )[ r0 + j ];
       if ( w == T( 0 ) )
         continue;
-      const uint32_t t = q.tdc[ r0 + j ];
-      const int dl = ( int ) ( ( t >> q.tbits ) & q.dmask );
-      if ( dl < q.d_lo || dl >= q.d_hi )
-        continue;
-      const unsigned l = ( t & q.tmask ) - ( unsigned ) q.a;
-      const unsigned own = l % ( unsigned ) q.G;
-      const unsigned cl = split && cell == OW_COUNT ? ( w < T( 0 ) ? 1u : 0u ) : t >> 31;
-      const long long e = s_base[ own ] + atomicAdd( &s_at[ warp ][ own ], 1u );
-      const uint32_t x = ( ( uint32_t ) dl * ( uint32_t ) nl + l / ( unsigned ) q.G ) | ( cl << 31 );
-      if ( cell == OW_I64 )
-        word_w[ e ] = make_uint2( x, ( uint32_t ) ( int ) w );
-      else if ( w16 )
-        reinterpret_cast< uint16_t* >( word )[ e ] = ( uint16_t ) ( ( x & 0x7fffu ) | ( cl << 15 ) );
+      uint32_t x;
+      const unsigned seg = own_place( q, q.tdc[ r0 + j ], w, q.split && CELL == OW_COUNT, nl, x );
+      const long long e = s_base[ seg ] + atomicAdd( &s_at[ warp ][ seg ], 1u );
+      if ( CELL == OW_I64 )
+        reinterpret_cast< uint2* >( word )[ e ] = make_uint2( x, ( uint32_t ) ( int ) w );
+      else if ( CELL == OW_COUNT && w16 )
+        reinterpret_cast< uint16_t* >( word )[ e ] = own_word16( x );
       else
       {
         word[ e ] = x;
-        if ( cell == OW_F64 )
+        if ( CELL == OW_F64 )
           weight[ e ] = ( double ) w;
       }
     }
     __syncwarp();
   }
+}
+
+// Bytes of a quad of edges in the staging buffer: words, and FP64 weights.
+__host__ __device__ inline int
+own_quad_bytes( int cell, int w16 )
+{
+  return cell == OW_I64 ? 32 : cell == OW_F64 ? 48 : w16 ? 8 : 16;
+}
+
+constexpr int OW_FILL_SMEM = 73728;  // three CTAs' staging buffers fit an SM
+
+// The same for long rows, a row per CTA: the row's segments are put together
+// in shared memory, padding included, and written out whole.  (Written edge by
+// edge, each to a sector of its own, 4.6e8 edges took 12.6 ms.)  Segments that
+// do not fit the buffer together are taken in rounds over the row, one that
+// does not fit it alone edge by edge.
+template < typename T, int CELL >
+__global__ void __launch_bounds__( 512 )
+k_own_fill_rows( OwnBuild q, int w16, int nl, uint32_t pad, const long long* e_near, const long long* e_far, uint32_t* word,
+  double* weight )
+{
+  extern __shared__ __align__( 16 ) unsigned char f_smem[];
+  __shared__ long long s_base[ 2 * OW_MAX_G ];   // a segment's first quad
+  __shared__ int s_p[ 2 * OW_MAX_G + 1 ];        // ... its place in the row's segments one after the other [quads]
+  __shared__ unsigned s_cnt[ 2 * OW_MAX_G ];
+  __shared__ int s_w[ 16 ];
+  static_assert( 2 * OW_MAX_G == 512, "a thread per segment" );
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G2 = q.rp_far ? 2 * q.G : q.G, cap = OW_FILL_SMEM / own_quad_bytes( CELL, w16 );
+  uint32_t* const b32 = reinterpret_cast< uint32_t* >( f_smem );
+  uint2* const b64 = reinterpret_cast< uint2* >( f_smem );
+  uint16_t* const b16 = reinterpret_cast< uint16_t* >( f_smem );
+  double* const bw = reinterpret_cast< double* >( f_smem + ( size_t ) cap * 16 );  // (OW_F64)
+  for ( long long s = blockIdx.x; s < q.n; s += gridDim.x )
+  {
+    int len = 0;
+    if ( tid < G2 )
+    {
+      const bool far = tid >= q.G;
+      const int c = q.c0 + ( far ? tid - q.G : tid );
+      const uint32_t* const rp = ( far ? q.rp_far : q.rp ) + q.rp_base[ c ] + s;
+      len = ( int ) ( rp[ 1 ] - rp[ 0 ] );
+      s_base[ tid ] = ( far ? e_far[ c ] : e_near[ c ] ) + rp[ 0 ];
+    }
+    int x = len;
+#pragma unroll
+    for ( int d = 1; d < 32; d <<= 1 )
+    {
+      const int y = __shfl_up_sync( FULL, x, d );
+      if ( lane >= d )
+        x += y;
+    }
+    if ( lane == 31 )
+      s_w[ warp ] = x;
+    __syncthreads();
+    for ( int k = 0; k < warp; ++k )
+      x += s_w[ k ];
+    s_p[ tid + 1 ] = x;
+    if ( tid == 0 )
+      s_p[ 0 ] = 0;
+    __syncthreads();
+    const long long r0 = q.row_beg[ q.a + s ];
+    const int deg = q.real_deg[ q.a + s ];
+    for ( int k0 = 0; k0 < G2; )
+    {
+      // segments k0 .. k1 - 1 fit the buffer together
+      int k1 = k0, hi = G2;
+      while ( k1 < hi )
+      {
+        const int mid = ( k1 + hi + 1 ) >> 1;
+        if ( s_p[ mid ] - s_p[ k0 ] <= cap )
+          k1 = mid;
+        else
+          hi = mid - 1;
+      }
+      const bool staged = k1 > k0;
+      if ( !staged )
+        k1 = k0 + 1;
+      const int p0 = s_p[ k0 ], nq = s_p[ k1 ] - p0;
+      if ( tid >= k0 && tid < k1 )
+        s_cnt[ tid ] = 0u;
+      if ( staged )
+      {
+        for ( int k = tid; k < 4 * nq; k += 512 )
+          if ( CELL == OW_I64 )
+            b64[ k ] = make_uint2( pad, 0u );
+          else if ( CELL == OW_COUNT && w16 )
+            b16[ k ] = ( uint16_t ) pad;
+          else
+          {
+            b32[ k ] = pad;
+            if ( CELL == OW_F64 )
+              bw[ k ] = 0.0;
+          }
+      }
+      __syncthreads();
+#pragma unroll 4
+      for ( int j = tid; j < deg; j += 512 )
+      {
+        const T w = ( ( const T* ) q.w )[ r0 + j ];
+        const uint32_t t = q.tdc[ r0 + j ];
+        if ( w == T( 0 ) )
+          continue;
+        uint32_t v;
+        const int seg = ( int ) own_place( q, t, w, q.split && CELL == OW_COUNT, nl, v );
+        if ( seg < k0 || seg >= k1 )
+          continue;
+        const unsigned at = atomicAdd( &s_cnt[ seg ], 1u );
+        if ( staged )
+        {
+          const unsigned e = 4u * ( unsigned ) ( s_p[ seg ] - p0 ) + at;
+          if ( CELL == OW_I64 )
+            b64[ e ] = make_uint2( v, ( uint32_t ) ( int ) w );
+          else if ( CELL == OW_COUNT && w16 )
+            b16[ e ] = own_word16( v );
+          else
+          {
+            b32[ e ] = v;
+            if ( CELL == OW_F64 )
+              bw[ e ] = ( double ) w;
+          }
+        }
+        else
+        {
+          const long long e = 4 * s_base[ seg ] + at;
+          if ( CELL == OW_I64 )
+            reinterpret_cast< uint2* >( word )[ e ] = make_uint2( v, ( uint32_t ) ( int ) w );
+          else if ( CELL == OW_COUNT && w16 )
+            reinterpret_cast< uint16_t* >( word )[ e ] = own_word16( v );
+          else
+          {
+            word[ e ] = v;
+            if ( CELL == OW_F64 )
+              weight[ e ] = ( double ) w;
+          }
+        }
+      }
+      __syncthreads();
+      if ( staged )
+      {
+        for ( int k = k0 + warp; k < k1; k += 16 )
+        {
+          const int l0 = s_p[ k ] - p0, n = s_p[ k + 1 ] - s_p[ k ];
+          const long long g0 = s_base[ k ];
+          if ( CELL == OW_COUNT && w16 )
+          {
+            for ( int u = lane; u < n; u += 32 )
+              reinterpret_cast< uint2* >( word )[ g0 + u ] = reinterpret_cast< const uint2* >( f_smem )[ l0 + u ];
+          }
+          else
+          {
+            constexpr int V = CELL == OW_I64 ? 2 : 1;  // 16-byte pieces of a quad's words
+            for ( int u = lane; u < V * n; u += 32 )
+              reinterpret_cast< uint4* >( word )[ V * g0 + u ] = reinterpret_cast< const uint4* >( f_smem )[ V * l0 + u ];
+            if ( CELL == OW_F64 )
+              for ( int u = lane; u < 2 * n; u += 32 )
+                reinterpret_cast< double2* >( weight )[ 2 * g0 + u ] = reinterpret_cast< const double2* >( bw )[ 2 * l0 + u ];
+          }
+        }
+      }
+      else
+        for ( long long e = 4 * s_base[ k0 ] + s_cnt[ k0 ] + tid; e < 4 * ( s_base[ k0 ] + nq ); e += 512 )
+        {
+          // the padding of a segment written edge by edge
+          if ( CELL == OW_I64 )
+            reinterpret_cast< uint2* >( word )[ e ] = make_uint2( pad, 0u );
+          else if ( CELL == OW_COUNT && w16 )
+            reinterpret_cast< uint16_t* >( word )[ e ] = ( uint16_t ) pad;
+          else
+          {
+            word[ e ] = pad;
+            if ( CELL == OW_F64 )
+              weight[ e ] = 0.0;
+          }
+        }
+      __syncthreads();  // (the buffer and counters are used again)
+      k0 = k1;
+    }
+  }
+}
+
+// The largest in-degree of a neuron and input class, from the owners' copies:
+// one CTA per owner counts its columns in shared memory (an L2 atomic per edge
+// as the rows are read took as long again as the reading).
+template < int CELL >
+__global__ void __launch_bounds__( 1024 )
+k_own_indeg( OwnNet o, const unsigned long long* total, unsigned* most )
+{
+  __shared__ unsigned s_h[ 2 ][ 2 * OW_TPB + 1 ];
+  for ( int k = threadIdx.x; k < 2 * OW_TPB + 1; k += blockDim.x )
+    s_h[ 0 ][ k ] = s_h[ 1 ][ k ] = 0u;
+  __syncthreads();
+  const bool w16 = CELL == OW_COUNT && o.w16;
+  for ( int f = 0; f <= o.far; ++f )
+  {
+    const long long base = f ? o.e_far[ blockIdx.x ] : o.e_base[ blockIdx.x ];
+    const long long n = ( long long ) total[ f * gridDim.x + blockIdx.x ];
+    for ( long long k = threadIdx.x; k < n; k += blockDim.x )
+    {
+      OwnQuad< CELL > x;
+      own_load< CELL >( o, base + k, x );
+#pragma unroll
+      for ( int e = 0; e < 4; ++e )
+        atomicAdd( &s_h[ w16 ? x.t[ e ] >> 15 : x.t[ e ] >> 31 ][ ( x.t[ e ] & ( w16 ? 0x7fffu : 0x7fffffffu ) ) % ( unsigned ) o.nl ],
+          1u );
+    }
+  }
+  __syncthreads();
+  unsigned m = 0;
+  for ( int k = threadIdx.x; k < o.nl - 1; k += blockDim.x )  // (column nl - 1: the segments' padding)
+    m = max( m, max( s_h[ 0 ][ k ], s_h[ 1 ][ k ] ) );
+  m = __reduce_max_sync( FULL, m );
+  if ( ( threadIdx.x & 31 ) == 0 && m )
+    atomicMax( most, m );
 }
 
 }  // namespace ng

@@ -150,3 +150,55 @@ def test_parts(n, nets):
     # no SM has much more than its share of the neurons
     assert f["own_neurons"] <= 2 * -(-n // f["own_ctas"])
     assert f["own_ctas"] >= 100
+
+
+# precision, one weight per class, longest delay (the last: 4-byte edge words), in-edges of target 3, cell
+@pytest.mark.parametrize("precision,uniform,maxd,many,cell", [
+    (_abi.NG_FP64, True, 15, 12000, COUNT), (_abi.NG_FP32, False, 15, 12000, FIXED), (_abi.NG_FP64, False, 15, 12000, F64),
+    (_abi.NG_FP32, True, 2500, 12000, COUNT), (_abi.NG_FP32, False, 15, 66000, None), (_abi.NG_FP64, False, 15, 66000, F64)])
+def test_long_rows(precision, uniform, maxd, many, cell):
+    """Rows whose segments are put together in shared memory: in one round, in
+    several (60,000 edges), one segment larger than the buffer (`many` edges of
+    one source to one target), sources without edges; and more in-edges than a
+    count or a fixed-point cell holds."""
+    n, md = 1103, 5
+
+    def run(variant):
+        rng = np.random.default_rng(9)
+        deg = rng.integers(1900, 2600, n)
+        deg[::50] = 0
+        deg[5], deg[7] = 60000, many + 40000
+        row = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+        src = np.repeat(np.arange(n), deg)
+        tgt = rng.integers(0, n, len(src)).astype(np.int32)
+        tgt[row[7]:row[7] + many] = 3
+        w = np.where(src % 5 < 4, 0.5, -2.0)
+        if not uniform:
+            w = w * rng.choice([1.0, 1.25, 0.0], len(src), p=[0.5, 0.45, 0.05])
+            w[row[7]:row[7] + many] = 0.25
+        eng = _abi.Engine([(_abi.NG_IAF_PSC_EXP, n)], 0.1, md, maxd, precision=precision)
+        eng.set_tuning(0, variant, -1, -1)
+        V = rng.uniform(0.0, 14.5, n)
+        V[[5, 7]] = 16.0
+        eng.set_var(0, "V_m_rel", V)
+        eng.set_connections(row, tgt, w, rng.integers(md, min(maxd, 60) + 1, len(src)).astype(np.int32))
+        eng.set_recording(np.ones(n, dtype=np.uint8))
+        eng.set_poisson(np.full(n, 11000.0), np.full(n, 48.0), np.full(n, md, dtype=np.int32), 0, 10**9, 3)
+        eng.simulate(300)
+        s, t = eng.spikes()
+        o = np.lexsort((s, t))
+        out = [s[o], t[o]] + [eng.get_var(0, v) for v in ("V_m_rel", "I_syn_ex", "I_syn_in")]
+        f = eng.slice_form()
+        eng.close()
+        return out, f
+
+    ref, got = run(0)[0], run(5)
+    assert len(ref[0]) > 100 and {5, 7} <= set(ref[0][:2])
+    for a, b in zip(ref, got[0]):
+        np.testing.assert_array_equal(a, b)
+    f = got[1]
+    if cell is None:
+        assert f["own_state"] == -1
+    else:
+        assert f["own_state"] == 1 and f["own_cell"] == cell and f["slices"]["k_run_owned"] == 60
+        assert f["own_edges"] >= 2048 * n
