@@ -299,6 +299,15 @@ int ng_get_tuning( ng_engine* eng, ng_tuning* out );
 #define NG_FORM_SCATTER_MG 3 /* k_run_slices_mg: the same for larger networks */
 #define NG_FORM_OWNED 4    /* k_run_owned: many slices in one launch, each SM owning its targets */
 
+/* NG_FORM_OWNED keeps a copy of the network's edges, grouped by the SM that owns
+ * their targets: 2 to 12 bytes per edge and 4 bytes per neuron and SM, held until the
+ * graph changes (serving engines: until the last network is removed) or another
+ * form is chosen.  It is built by ng_simulate (100 us below 1e5 edges, some 0.7 ms
+ * plus 45 us per 1e6 edges, 9 ms at 4.6e8) once the slices run since the graph
+ * changed, with the call's, repay it -- 15 slices below 1e5 edges, 100 to 300
+ * above -- and at once where ng_set_tuning fixed update variant 5; shorter calls
+ * and networks without the memory for it run in the other forms. */
+
 /* Which form ran, and the target-owning kernel's layout for the network as it
  * is connected now (own_* below it are those of the last layout built). */
 typedef struct

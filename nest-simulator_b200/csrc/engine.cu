@@ -757,6 +757,8 @@ struct ng_engine
   size_t own_smem_bytes = 0;
   OwnNet own_net_d {};
   uint64_t own_seq = 0;      // slices published so far (tags of the exchange buffer)
+  int64_t own_ran = 0;       // slices that calls of many ran in other forms since the graph changed
+  bool own_call = false;     // this call's full slices go to the owning kernel
   int own_n_parts = 0, own_n_loc = 0;
   int64_t own_edges = 0, own_far_edges = 0;
   // full slices run so far, by form, and the last one's form (ng_get_slice_form)
@@ -1390,8 +1392,8 @@ struct ng_engine
     return *n <= ( int64_t ) sms * 2 * OW_TPB && *n < ( 1 << OW_SBITS ) && sms <= OW_MAX_G;
   }
 
-  // the owners' layout: built at the first call after the graph changed.  A
-  // network it does not suit (or that does not fit) keeps the other kernels.
+  // the owners' layout, built now if it is not yet.  A network it does not suit
+  // (or that does not fit) keeps the other kernels.
   bool
   own_ready()
   {
@@ -1403,9 +1405,91 @@ struct ng_engine
     {
       own_state = own_build( a, n, id ) == NG_OK ? 1 : -1;
       if ( own_state < 0 )
+      {
         cudaGetLastError();
+        own_release();
+      }
     }
     return own_state > 0;
+  }
+
+  // the graph changed: the layout is stale (its buffers may serve the next one)
+  void
+  own_forget()
+  {
+    own_state = 0;
+    own_ran = 0;
+    own_call = false;
+  }
+
+  void
+  own_release()
+  {
+    for ( DevBuf* b : { &own_tab, &own_word, &own_tmp } )
+      release( *b );
+    own_x = nullptr;
+  }
+
+  // another form was chosen: the layout's memory goes back
+  void
+  own_drop_unused()
+  {
+    if ( upd_variant >= 0 && upd_variant != 5 && own_state > 0 )
+    {
+      own_forget();
+      own_release();
+    }
+  }
+
+  // full slices that repay a build.  It takes [us] 100 below 1e5 edges, else
+  // 700 (two allocations) and 45 per 1e6 edges, 17 from 5e7 edges on (long rows);
+  // a slice is faster than by the kernels per slice, which run meanwhile, by 7
+  // and by 1 per 4e6 edges, up to 35.  Measured: 1,000 neurons x 100 100 and 7.7,
+  // 4,000 x 400 800 and 7.6, 12,500 x 1,250 1,300 and 19, 30,000 x 1,250 2,300
+  // and 25, layered network at 1/4 1,400 and 14, at 1/2 3,500, full 9,200 and
+  // 31 to 46.
+  static int64_t
+  own_repay( int64_t edges )
+  {
+    const double m = 1e-6 * ( double ) edges;
+    const double build = edges < 100000 ? 100.0 : 700.0 + ( m < 50.0 ? 45.0 * m : 2250.0 + 17.0 * ( m - 50.0 ) );
+    return ( int64_t ) ( build / ( 7.0 + std::min( 0.25 * m, 28.0 ) ) );
+  }
+
+  int64_t
+  own_edges_of( int id ) const
+  {
+    return id >= 0 ? nets[ ( size_t ) id ].ne : nnz_padded;
+  }
+
+  // a serving engine's network runs long enough to repay a build
+  bool
+  own_lives( int id ) const
+  {
+    return id < 0 || ( nets[ ( size_t ) id ].until - origin ) / cfg.min_delay >= own_repay( own_edges_of( id ) );
+  }
+
+  // does a call of `full` full slices go to the owning kernel?  Decided once
+  // per call: the layout is built here when the slices that ran without it
+  // since the graph changed, with this call's, repay it (and a serving
+  // engine's network lives that long), at once where the caller fixed the
+  // persistent form.
+  bool
+  own_take( int64_t full )
+  {
+    int64_t a = 0, n = 0;
+    int id = -1;
+    if ( ( upd_variant >= 0 && upd_variant != 5 ) || own_state < 0 || full < 2 || !own_possible( &a, &n, &id ) )
+      return false;
+    if ( own_state == 0 && !( tune_mode == 0 && upd_variant == 5 ) )
+    {
+      if ( own_ran + full < own_repay( own_edges_of( id ) ) || !own_lives( id ) )
+      {
+        own_ran += full;
+        return false;
+      }
+    }
+    return own_ready();
   }
 
   // Contiguous, mutually unconnected parts of the network (the copies of a
@@ -1798,9 +1882,11 @@ struct ng_engine
   // full slices the target-owning kernel may run from here on (0: none): a
   // serving engine's network must live through all of them
   int64_t
-  own_slices( int64_t full )
+  own_slices( int64_t full ) const
   {
-    if ( full < 1 || !own_ready() )
+    int64_t a = 0, n = 0;
+    int id = -1;
+    if ( full < 1 || own_state <= 0 || !own_possible( &a, &n, &id ) )
       return 0;
     if ( own_net >= 0 )
       full = std::min< int64_t >( full, ( nets[ ( size_t ) own_net ].until - origin ) / cfg.min_delay );
@@ -2160,15 +2246,15 @@ struct ng_engine
     const Net d = net();
     while ( n > 0 )
     {
-      // the persistent forms: the target-owning kernel where the network
-      // suits it -- also before tuning -- else the scatter form.  A single
+      // the persistent forms: the target-owning kernel in calls that own_take
+      // gave it -- also before tuning -- else the scatter form.  A single
       // slice (a node's call per slice) does not repay the owning kernel's
       // prologue and epilogue: 43 against 21 us per call at 12,500 neurons
       // (one-wave scatter form), 54 against 25 at 19,300 (graph).
       const int64_t full = from == 0 ? n / cfg.min_delay : 0;
-      const int64_t owned = ( upd_variant == 5 || upd_variant < 0 ) && full > 1 ? own_slices( full ) : 0;
+      const int64_t owned = own_call && full > 1 ? own_slices( full ) : 0;
       const bool scatter = owned == 0 && upd_variant == 5 && full > 0 && persistent_ok()
-        && ( full > 1 || !pk_multi_group() || !own_ready() );
+        && ( full > 1 || !pk_multi_group() || own_state <= 0 );
       if ( owned > 0 || scatter )
       {
         const int k = ( int ) std::min< int64_t >( owned > 0 ? owned : full, 1 << 20 );
@@ -2581,6 +2667,7 @@ struct ng_engine
         return rc;
       }
     }
+    own_call = false;
     if ( ( rc = enqueue_steps( to_ - from_ ) ) )
       return rc;
     og_steps += to_ - from_;
@@ -2679,6 +2766,24 @@ struct ng_engine
     for ( const auto& b : blk )
       iaf = iaf || b.model != NG_AEIF_COND_ALPHA;
     std::vector< int > variants;
+    // A network that k_run_owned takes runs in it without trials.  It was the
+    // fastest form of every such network measured, from 100 neurons of 12
+    // inputs to 150,000 of 60 (one call of 1 s or 0.6 s, it against the best
+    // of the others [ms]: 100 x 12 3.2 / 8.7, 20,000 x 60 10.5 / 20.1, 20,000 x
+    // 200 9.9 / 18.5, 100,000 x 100 32.9 / 44.5, 100,000 x 1,000 15.1 / 26.5,
+    // 150,000 x 60 56.9 / 67.1), and trials of few steps can choose wrongly:
+    // in the layered network of 77,169 neurons, which alternates between
+    // silence and bursts, a group of 9 steps took from 29 to 190 us per step
+    // with one and the same form, and trials of 4 slices charge each the
+    // prologue of a call.  Until its slices repay the layout it waits for that,
+    // untuned; a serving engine stays untuned, for the networks to come.
+    int64_t own_a = 0, own_n = 0;
+    int own_id = -1;
+    const bool own_suits = own_state >= 0 && own_possible( &own_a, &own_n, &own_id );
+    const bool own_rule = tune_mode == 1 && own_suits && ( own_state > 0 || own_lives( own_id ) );
+    if ( own_rule && ( serving || !own_call ) )
+      return NG_OK;
+    const bool own_trial = tune_mode == 2 && own_suits;
     if ( iaf )
     {
       variants = { 0, 1, 6 };
@@ -2687,7 +2792,7 @@ struct ng_engine
         variants.push_back( 2 );
         variants.push_back( 3 );
       }
-      if ( own_ready() || persistent_ok() )
+      if ( own_call || own_trial || persistent_ok() )
         variants.push_back( 5 );
     }
     std::vector< int > per_sm;
@@ -2708,6 +2813,12 @@ struct ng_engine
       gmax / md } );
     if ( S < 4 )
       return NG_OK;
+    if ( own_trial )
+    {
+      own_call = own_ready();  // the trial of variant 5 runs in it
+      if ( !own_call && !persistent_ok() )
+        variants.pop_back();
+    }
     const int64_t steps = S * md;
     const int v0 = upd_variant >= 0 ? upd_variant : ( iaf ? engine_default_variant( blk[ 0 ].n ) : 0 );
     TuneCand best { v0, deliver_per_sm, deliver_group, 1e300 };
@@ -2746,20 +2857,11 @@ struct ng_engine
       {
         apply_cand( it->second );
         tune_state = 2;
+        own_drop_unused();
         return NG_OK;
       }
     }
-    // A static network that k_run_owned takes runs in it without trials (a
-    // serving engine, tuned on request only, measures).  It was the
-    // fastest form of every such network measured, from 100 neurons of 12
-    // inputs to 150,000 of 60 (one call of 1 s or 0.6 s, it against the best
-    // of the others [ms]: 100 x 12 3.2 / 8.7, 20,000 x 60 10.5 / 20.1, 20,000 x
-    // 200 9.9 / 18.5, 100,000 x 100 32.9 / 44.5, 100,000 x 1,000 15.1 / 26.5,
-    // 150,000 x 60 56.9 / 67.1), and trials of few steps can choose wrongly:
-    // in the layered network of 77,169 neurons, which alternates between
-    // silence and bursts, a group of 9 steps took from 29 to 190 us per step
-    // with one and the same form.
-    if ( tune_mode == 1 && !serving && own_ready() )
+    if ( own_rule )
     {
       apply_cand( TuneCand { 5, deliver_per_sm, deliver_group, 0.0 } );
       tune_state = 1;
@@ -2801,6 +2903,7 @@ struct ng_engine
     }
     apply_cand( best );
     tune_state = 1;
+    own_drop_unused();
     {
       std::lock_guard< std::mutex > lock( tune_mutex() );
       tune_cache()[ key ] = best;
@@ -2848,6 +2951,7 @@ struct ng_engine
       if ( quarter >= q && quarter < gmax )
         gmax = quarter;
     }
+    own_call = own_take( ( n - ( from ? cfg.min_delay - from : 0 ) ) / cfg.min_delay );
     // the autotuner runs on the first long enough call, at a slice boundary,
     // with no group in flight and no tracing or profiling
     bool live = nnz_padded > 0;
@@ -3323,6 +3427,9 @@ ng_set_connections( ng_engine* e, int64_t n_src, const int64_t* row_ptr, const i
   if ( row_ptr[ 0 ] != 0 || nnz < 0 || ( nnz > 0 && ( !target || !weight || !delay_steps ) ) )
     return fail( NG_ERR_ARG, "ng_set_connections: bad CSR" );
   cudaSetDevice( e->cfg.device );
+  // the owning kernel's copies of the graph that is replaced
+  e->own_forget();
+  e->own_release();
   std::vector< int64_t > prow( ( size_t ) n_src + 1, 0 );
   std::vector< int32_t > rdeg( ( size_t ) n_src, 0 );
   for ( int64_t s = 0; s < n_src; ++s )
@@ -3427,7 +3534,6 @@ ng_set_connections( ng_engine* e, int64_t n_src, const int64_t* row_ptr, const i
   free_tmp();
   e->fx_inv = fx ? std::ldexp( 1.0, -S ) : 1.0;
   e->nnz_padded = np;
-  e->own_state = 0;
   e->chunks_all_src = 0;
   e->chunks_max_gen = 0;
   for ( int64_t sidx = 0; sidx < n_src; ++sidx )
@@ -3998,6 +4104,7 @@ ng_set_tuning( ng_engine* e, int32_t mode, int32_t update_variant, int32_t deliv
     e->deliver_per_sm = deliver_ctas_per_sm > 0 ? std::min( deliver_ctas_per_sm, e->occ_deliver ) : e->occ_deliver;
     e->deliver_group = deliver_chunks_per_warp > 0 ? deliver_chunks_per_warp : 4;
     e->tune_state = 3;
+    e->own_drop_unused();
   }
   else
   {
@@ -4715,7 +4822,7 @@ ng_net_add( ng_engine* e, const ng_net_desc* desc, int32_t* net_id )
   nw.sn = sgn;
   nw.step0 = step0;
   nw.until = until;
-  e->own_state = 0;
+  e->own_forget();
   nw.rec = desc->record != 0;
   nw.log_rate = desc->record ? log_rate : 0.0;
   e->n_rec += desc->record ? n : 0;
@@ -4953,9 +5060,13 @@ ng_net_remove( ng_engine* e, int32_t id )
   }
   e->n_rec -= nw.rec ? nw.n : 0;
   e->log_per_step = std::max( 1.0, e->log_per_step - nw.log_rate );
-  e->own_state = 0;
+  e->own_forget();
   ng_engine::free_blocks( nw.blocks );
   nw = ng_engine::NetInfo();
+  // with the last network the owning kernel's copies go too (kept between
+  // networks they would be allocated anew, a device-wide wait, beside others)
+  if ( std::none_of( e->nets.begin(), e->nets.end(), []( const ng_engine::NetInfo& x ) { return x.used; } ) )
+    e->own_release();
   e->refresh_late();
   return NG_OK;
 }

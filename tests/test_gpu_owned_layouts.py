@@ -202,3 +202,93 @@ def test_long_rows(precision, uniform, maxd, many, cell):
     else:
         assert f["own_state"] == 1 and f["own_cell"] == cell and f["slices"]["k_run_owned"] == 60
         assert f["own_edges"] >= 2048 * n
+
+
+def _plain(n, deg, md, seed=4, **kw):
+    rng = np.random.default_rng(seed)
+    eng = _abi.Engine([(_abi.NG_IAF_PSC_EXP, n)], 0.1, md, md, **kw)
+    _connect(eng, n, deg, md, seed)
+    eng.set_var(0, "V_m_rel", rng.uniform(0.0, 14.5, n))
+    eng.set_recording(np.ones(n, dtype=np.uint8))
+    eng.set_poisson(np.full(n, 11000.0), np.full(n, 48.0), np.full(n, md, dtype=np.int32), 0, 10**9, 3)
+    return eng
+
+
+def _connect(eng, n, deg, md, seed):
+    rng = np.random.default_rng(seed)
+    src = np.repeat(np.arange(n), deg)
+    eng.set_connections(np.arange(n + 1, dtype=np.int64) * deg, rng.integers(0, n, n * deg).astype(np.int32),
+                        np.where(src % 5 < 4, 60.0, -240.0), np.full(n * deg, md, dtype=np.int32))
+
+
+def _raster(eng):
+    s, t = eng.spikes()
+    o = np.lexsort((s, t))
+    return s[o], t[o], eng.get_var(0, "V_m_rel")
+
+
+def test_layout_waits_until_it_pays():
+    """Short calls on a new network build nothing; once the slices that ran
+    would have repaid the build it is there; a new graph starts over, and its
+    memory is given back; the results are those of one long call's form."""
+    n, deg, md = 4001, 60, 15
+    eng = _plain(n, deg, md)
+    own = lambda: eng.slice_form()["slices"]["k_run_owned"]  # noqa: E731
+    for k in (1, 15, 30, 60):
+        eng.simulate(k)
+        assert eng.slice_form()["own_state"] == 0 and eng.slice_form()["own_bytes"] == 0
+    for _ in range(40):
+        eng.simulate(20 * md)
+        if own():
+            break
+    ran = sum(eng.slice_form()["slices"].values())
+    assert own() > 0 and 60 < ran < 300
+    assert eng.slice_form()["own_bytes"] > 2 * n * deg
+    eng.simulate(14)                      # to the slice boundary again: 106 + 14 = 8 * 15
+    first = _raster(eng)
+    eng.simulate(9 * md)
+    _connect(eng, n, deg, md, 5)
+    f = eng.slice_form()
+    assert f["own_state"] == 0 and f["own_bytes"] == 0
+    eng.simulate(20 * md)
+    assert eng.slice_form()["own_state"] == 0
+    eng.simulate(600 * md)
+    assert eng.slice_form()["own_state"] == 1
+    second = _raster(eng)
+    eng.set_tuning(0, 2, -1, -1)          # another form is chosen: the memory goes back
+    assert eng.slice_form()["own_bytes"] == 0
+    eng.close()
+    ref = _plain(n, deg, md)
+    ref.set_tuning(0, 0, -1, -1)
+    steps = sum((1, 15, 30, 60)) + 14 + (ran - 7) * md
+    ref.simulate(steps)
+    for a, b in zip(first, _raster(ref)):
+        np.testing.assert_array_equal(a, b)
+    ref.simulate(9 * md)
+    _connect(ref, n, deg, md, 5)
+    ref.simulate(620 * md)
+    for a, b in zip(second, _raster(ref)):
+        np.testing.assert_array_equal(a, b)
+    ref.close()
+
+
+def test_serving_network_that_ends_soon_builds_nothing():
+    """A network that does not live long enough keeps the kernels per slice; a
+    longer one gets the layout, and the memory goes with the last network."""
+    from nestgpu import workloads
+
+    spec = workloads.layered_spec(seed=3, scale=0.05)
+    eng = workloads.layered_engine(spec, "fp64")
+    nid = workloads.layered_add(eng, spec, 40)
+    eng.simulate(40)
+    f = eng.slice_form()
+    assert f["slices"]["kernels"] == 40 and f["own_state"] == 0 and f["own_bytes"] == 0
+    eng.net_remove(nid)
+    nid = workloads.layered_add(eng, spec, 5000)
+    for _ in range(20):
+        eng.simulate(100)
+    f = eng.slice_form()
+    assert f["own_state"] == 1 and f["slices"]["k_run_owned"] >= 1500 and f["own_bytes"] > 0
+    eng.net_remove(nid)
+    assert eng.slice_form()["own_bytes"] == 0
+    eng.close()
