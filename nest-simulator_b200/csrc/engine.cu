@@ -1456,6 +1456,24 @@ struct ng_engine
     return ( int64_t ) ( build / ( 7.0 + std::min( 0.25 * m, 28.0 ) ) );
   }
 
+  // fewest full slices of a call that the owning kernel runs faster than the
+  // form it would else take: its prologue and epilogue (state, row tables and
+  // ring cells in and out) cost 20 to 25 us.  Calls of k slices, it against the
+  // other [us]: one-wave scatter form, 12,500 neurons k = 6 118 / 112, 8 130 / 136;
+  // 4,000 k = 2 68 / 61, 3 69 / 74; 1,000 k = 2 60 / 61; its multi-group form,
+  // 30,000 k = 4 149 to 158 / 147 to 151, 5 161 to 174 / 176 to 179; kernels per
+  // slice, 4,000 k = 2 70 / 63, 3 73 / 82; 30,000 k = 2 132 / 109, 3 145 / 150;
+  // layered network, full size k = 2 276 / 262, 3 334 / 372.
+  int64_t
+  own_min_slices( int64_t n )
+  {
+    if ( n < 2000 )
+      return 2;
+    if ( upd_variant != 5 || !persistent_ok() || n < 5000 )
+      return 3;
+    return pk_multi_group() ? 5 : 7;
+  }
+
   int64_t
   own_edges_of( int id ) const
   {
@@ -1479,7 +1497,8 @@ struct ng_engine
   {
     int64_t a = 0, n = 0;
     int id = -1;
-    if ( ( upd_variant >= 0 && upd_variant != 5 ) || own_state < 0 || full < 2 || !own_possible( &a, &n, &id ) )
+    if ( ( upd_variant >= 0 && upd_variant != 5 ) || own_state < 0 || full < 2 || !own_possible( &a, &n, &id )
+      || full < own_min_slices( n ) )
       return false;
     if ( own_state == 0 && !( tune_mode == 0 && upd_variant == 5 ) )
     {
@@ -2247,14 +2266,15 @@ struct ng_engine
     while ( n > 0 )
     {
       // the persistent forms: the target-owning kernel in calls that own_take
-      // gave it -- also before tuning -- else the scatter form.  A single
-      // slice (a node's call per slice) does not repay the owning kernel's
-      // prologue and epilogue: 43 against 21 us per call at 12,500 neurons
-      // (one-wave scatter form), 54 against 25 at 19,300 (graph).
+      // gave it -- also before tuning -- else the scatter form.  Of single slices
+      // (a node's call per slice, [us] scatter form / kernels per slice) the
+      // latter is the slower form in FP64 (18,900 neurons 28.6 / 42.9, 30,000 33.6 /
+      // 39.5, 60,000 49.0 / 63.9) and in FP32 up to some 50,000 neurons (30,000 34.8 /
+      // 44.4, 60,000 48.8 / 47.5, 100,000 46.0 / 38.6).
       const int64_t full = from == 0 ? n / cfg.min_delay : 0;
       const int64_t owned = own_call && full > 1 ? own_slices( full ) : 0;
       const bool scatter = owned == 0 && upd_variant == 5 && full > 0 && persistent_ok()
-        && ( full > 1 || !pk_multi_group() || own_state <= 0 );
+        && ( full > 1 || prec == NG_FP64 || N < 50000 );
       if ( owned > 0 || scatter )
       {
         const int k = ( int ) std::min< int64_t >( owned > 0 ? owned : full, 1 << 20 );

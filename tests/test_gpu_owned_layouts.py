@@ -246,7 +246,13 @@ def test_layout_waits_until_it_pays():
     assert eng.slice_form()["own_bytes"] > 2 * n * deg
     eng.simulate(14)                      # to the slice boundary again: 106 + 14 = 8 * 15
     first = _raster(eng)
-    eng.simulate(9 * md)
+    # short calls of a network whose layout is there: one and two slices take the other forms
+    before = own()
+    eng.simulate(md)
+    eng.simulate(2 * md)
+    assert own() == before
+    eng.simulate(6 * md)
+    assert own() == before + 6
     _connect(eng, n, deg, md, 5)
     f = eng.slice_form()
     assert f["own_state"] == 0 and f["own_bytes"] == 0
