@@ -562,7 +562,8 @@ ng_simulate_noalloc( const ng_noalloc_net* net, int64_t n_steps, void* cuda_stre
     int clusters = 0;
     const bool ok = cudaFuncSetAttribute( k_na_run, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 ) == cudaSuccess
       && cudaOccupancyMaxActiveClusters( &clusters, k_na_run, &lc ) == cudaSuccess && clusters > 0;
-    cudaGetLastError();  // (a refusal leaves no error behind)
+    if ( !ok )
+      cudaGetLastError();  // (a refusal leaves no error behind)
     g_na_cluster[ dev ] = ok ? 1 : -1;
   }
   if ( net->n <= NA_CL_CTAS * NA_CL_TPB && g_na_cluster[ dev ] > 0 )
@@ -573,6 +574,7 @@ ng_simulate_noalloc( const ng_noalloc_net* net, int64_t n_steps, void* cuda_stre
            net->continue_run ? 0 : 1 )
       != cudaSuccess )
     {
+      cudaGetLastError();
       ng_internal_set_error( "ng_simulate_noalloc: kernel launch failed" );
       return NG_ERR_CUDA;
     }

@@ -298,3 +298,33 @@ def test_serving_network_that_ends_soon_builds_nothing():
     eng.net_remove(nid)
     assert eng.slice_form()["own_bytes"] == 0
     eng.close()
+
+
+@pytest.mark.parametrize("rates,one_weight,own", [
+    (np.array([8e5]), True, True),                   # counts beyond the tabulated inputs, tables that are bisected
+    (np.array([8e5, 0.0, 5e3]), False, True),        # ... with weights of their own, neurons without drive
+    (np.linspace(1e3, 9e5, 40), True, True),         # more thresholds than shared memory holds
+    (np.array([8e5, 1.1e6]), True, False),           # a mean too large for a table: the other forms
+])
+@pytest.mark.parametrize("precision", [_abi.NG_FP64, _abi.NG_FP32])
+def test_drive_tables(rates, one_weight, own, precision):
+    n, md = 997, 10
+    idx = np.arange(n)
+
+    def run(variant):
+        eng = _plain(n, 20, md, precision=precision)
+        eng.set_tuning(0, variant, -1, -1)
+        w = np.full(n, 0.25) if one_weight else np.choose(idx % 3, [0.25, 0.5, -0.25])
+        eng.set_poisson(rates[idx % len(rates)], w, np.full(n, md, dtype=np.int32), 3, 10**9, 21)
+        eng.simulate(40 * md)
+        st = eng.stats()
+        out = _raster(eng) + (eng.get_var(0, "I_syn_ex"), eng.get_var(0, "I_syn_in"), np.array([st["drive_events"]]))
+        f = eng.slice_form()
+        eng.close()
+        return out, f
+
+    ref, got = run(0)[0], run(5)
+    assert len(ref[0]) > 100 and ref[-1][0] > 10 * n
+    for a, b in zip(ref, got[0]):
+        np.testing.assert_array_equal(a, b)
+    assert (got[1]["slices"]["k_run_owned"] == 40) == own
