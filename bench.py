@@ -65,7 +65,8 @@ def headline_config(ws):
     same network, form and simulated time per step."""
     return {"workload": WORKLOAD, "form": "plain FP64 (state, coefficients and ring buffers in FP64)",
             "networks_per_gpu": 1, "sim_ms_per_step": SIM_MS, "parallelism": f"replicas{ws}",
-            "l2": "graph (188 MB of edges) larger than L2: no flush needed"}
+            "l2": "flushed before every step by a 256 MB write inside the timed region (the kernel's own copy of the "
+                  "edges, 33 MB of 2-byte words, would else stay in L2)"}
 
 
 def cpu_model():
@@ -406,7 +407,9 @@ def measure(args, nest, KERNEL, form, precision, copies, seed, local, dev, pg, e
     eng = KERNEL.engine
     stream = torch.cuda.current_stream(dev)
     eng.set_stream(stream.cuda_stream)
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     for _ in range(args.warmup):
+        flush.zero_()
         nest.Run(SIM_MS)
     s0 = eng.stats()
     sampler = ClockSampler(local)
@@ -418,6 +421,7 @@ def measure(args, nest, KERNEL, form, precision, copies, seed, local, dev, pg, e
     e_end = torch.cuda.Event(enable_timing=True)
     e_start.record(stream)
     for _ in range(args.steps):
+        flush.zero_()
         nest.Run(SIM_MS)
     KERNEL.settle()  # the last Run's spikes reach the recorders inside the timed region
     e_end.record(stream)
@@ -456,7 +460,20 @@ def measure(args, nest, KERNEL, form, precision, copies, seed, local, dev, pg, e
 
     tuned = eng.tuned()
     upd_name = tuned.get("update_kernel", "k_update_iaf")
-    if upd_name in ("k_run_slices", "k_run_slices_mg", "k_run_owned"):
+    if upd_name == "k_run_owned":
+        # ring cells and state stay on chip for the launch: an event reads its
+        # edge word (and weight) from the owners' copies, a spike costs every SM
+        # of its network an exchange word and two row entries, and a log entry
+        sl = (p1["slices"] - p0["slices"]) / max(1, n_upd)
+        f = eng.slice_form()
+        fits = (c["max_delay"] + 1) * (f["own_neurons"] + 1) < 32768
+        b_event = {0: 2 if fits else 4, 1: 8, 2: 12}[f["own_cell"]]
+        per_spike = 16.0 * f["own_ctas"] / max(1, f["own_parts"]) + 16.0
+        b = N * B_NEURON_LAUNCH[precision] + (ev_prof * b_event + (p1["spikes"] - p0["spikes"]) * per_spike) / max(1, n_upd)
+        kernels = {upd_name: kern(n_upd, upd_ms, b, b)}
+        kernels[upd_name]["slices_per_launch"] = sl
+        kernels[upd_name]["bytes_per_event"] = b_event
+    elif upd_name in ("k_run_slices", "k_run_slices_mg"):
         # one launch runs node update and delivery of many slices: its bytes are
         # both phases' for every slice it covers
         sl = (p1["slices"] - p0["slices"]) / max(1, n_upd)
@@ -942,8 +959,12 @@ def run_engine(args):
         "clocks": r["clocks"],
         "roofline": {"bound": "hbm", "kernel": dom_name, "achieved": ach, "peak": peak, "unit": "GB/s",
                      "frac": (ach / peak) if ach else None, "peak_kind": peak_kind,
-                     "bytes_model": "per-unit bytes of the path's survey: 96 B per iaf_psc_exp neuron-step "
-                                    "(FP64), 29 B per synaptic event",
+                     "bytes_model": (f"what the kernel reads: {dom['bytes_per_event']} B per synaptic event, state once per "
+                                     "launch, exchange words and row entries per spike; it is bound by the serial chain "
+                                     "of a slice (inputs, recurrence, exchange, delivery), not by memory"
+                                     if "bytes_per_event" in dom else
+                                     "per-unit bytes of the path's survey: 96 B per iaf_psc_exp neuron-step "
+                                     "(FP64), 29 B per synaptic event"),
                      "frac_engine_model": (dom["engine_model_gbs"] / peak) if dom["engine_model_gbs"] else None,
                      "traffic": load_traffic(dom_name, "brunel_x1_fp64", dom.get("slices_per_launch")),
                      "kernels": r["kernels"]},
