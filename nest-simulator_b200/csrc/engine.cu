@@ -2787,8 +2787,9 @@ struct ng_engine
       iaf = iaf || b.model != NG_AEIF_COND_ALPHA;
     std::vector< int > variants;
     // A network that k_run_owned takes runs in it without trials.  It was the
-    // fastest form of every such network measured, from 100 neurons of 12
-    // inputs to 150,000 of 60 (one call of 1 s or 0.6 s, it against the best
+    // fastest form of every such network measured (what it is not the fastest
+    // form of, it refuses: own_far_pays), from 100 neurons of 12 inputs to
+    // 150,000 of 60 (one call of 1 s or 0.6 s, it against the best
     // of the others [ms]: 100 x 12 3.2 / 8.7, 20,000 x 60 10.5 / 20.1, 20,000 x
     // 200 9.9 / 18.5, 100,000 x 100 32.9 / 44.5, 100,000 x 1,000 15.1 / 26.5,
     // 150,000 x 60 56.9 / 67.1), and trials of few steps can choose wrongly:
