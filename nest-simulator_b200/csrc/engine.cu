@@ -1497,8 +1497,9 @@ struct ng_engine
   {
     int64_t a = 0, n = 0;
     int id = -1;
-    if ( ( upd_variant >= 0 && upd_variant != 5 ) || own_state < 0 || full < 2 || !own_possible( &a, &n, &id )
-      || full < own_min_slices( n ) )
+    // (a choice of the autotuner that is still to come overrides an earlier fixed variant)
+    const bool other = upd_variant >= 0 && upd_variant != 5 && ( tune_mode == 0 || tune_state != 0 );
+    if ( other || own_state < 0 || full < 2 || !own_possible( &a, &n, &id ) || full < own_min_slices( n ) )
       return false;
     if ( own_state == 0 && !( tune_mode == 0 && upd_variant == 5 ) )
     {

@@ -328,3 +328,22 @@ def test_drive_tables(rates, one_weight, own, precision):
     for a, b in zip(ref, got[0]):
         np.testing.assert_array_equal(a, b)
     assert (got[1]["slices"]["k_run_owned"] == 40) == own
+
+
+def test_automatic_choice_after_a_fixed_one():
+    eng = _plain(2503, 30, 15)
+    eng.set_tuning(0, 2, -1, -1)
+    eng.simulate(300)
+    assert eng.slice_form()["slices"]["k_run_owned"] == 0
+    eng.set_tuning(1)
+    eng.simulate(6000)
+    f, t = eng.slice_form(), eng.tuned()
+    got = _raster(eng)
+    eng.close()
+    assert f["slices"]["k_run_owned"] == 400 and t["state"] == "tuned" and t["update_variant"] == 5
+    ref = _plain(2503, 30, 15)
+    ref.set_tuning(0, 0, -1, -1)
+    ref.simulate(6300)
+    for a, b in zip(got, _raster(ref)):
+        np.testing.assert_array_equal(a, b)
+    ref.close()
