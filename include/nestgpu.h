@@ -304,7 +304,7 @@ int ng_get_tuning( ng_engine* eng, ng_tuning* out );
  * graph changes (serving engines: until the last network is removed) or another
  * form is chosen.  It is built by ng_simulate (100 us below 1e5 edges, some 0.7 ms
  * plus 45 us per 1e6 edges, 9 ms at 4.6e8) once the slices run since the graph
- * changed, with the call's, repay it -- 15 slices below 1e5 edges, 100 to 300
+ * changed, with the call's, repay it -- 15 slices below 1e5 edges, 50 to 250
  * above -- and at once where ng_set_tuning fixed update variant 5; shorter calls
  * and networks without the memory for it run in the other forms. */
 

@@ -1442,18 +1442,19 @@ struct ng_engine
   }
 
   // full slices that repay a build.  It takes [us] 100 below 1e5 edges, else
-  // 700 (two allocations) and 45 per 1e6 edges, 17 from 5e7 edges on (long rows);
-  // a slice is faster than by the kernels per slice, which run meanwhile, by 7
-  // and by 1 per 4e6 edges, up to 35.  Measured: 1,000 neurons x 100 100 and 7.7,
-  // 4,000 x 400 800 and 7.6, 12,500 x 1,250 1,300 and 19, 30,000 x 1,250 2,300
-  // and 25, layered network at 1/4 1,400 and 14, at 1/2 3,500, full 9,200 and
-  // 31 to 46.
-  static int64_t
-  own_repay( int64_t edges )
+  // 700 (an allocation of more than 1 MB, or two) and 45 per 1e6 edges, 17 from
+  // 5e7 edges on (long rows).  A slice is faster than by the kernels per slice,
+  // which run meanwhile, by 7 (by 12 where it has one or two steps, which the
+  // one-thread update serves) and by 1 per 4e6 edges, up to 28.  Measured, build
+  // and gain: 1,000 neurons x 100 100 and 7.7, 4,000 x 400 500 and 7.6, 12,500 x 1,250
+  // 1,300 and 19, 30,000 x 1,250 2,300 and 25; single steps: layered network at
+  // 0.14 1,100 and 14, at 1/4 1,400 and 14, full 9,200 and 31 to 46.
+  int64_t
+  own_repay( int64_t edges ) const
   {
     const double m = 1e-6 * ( double ) edges;
     const double build = edges < 100000 ? 100.0 : 700.0 + ( m < 50.0 ? 45.0 * m : 2250.0 + 17.0 * ( m - 50.0 ) );
-    return ( int64_t ) ( build / ( 7.0 + std::min( 0.25 * m, 28.0 ) ) );
+    return ( int64_t ) ( build / ( ( cfg.min_delay <= 2 ? 12.0 : 7.0 ) + std::min( 0.25 * m, 28.0 ) ) );
   }
 
   // fewest full slices of a call that the owning kernel runs faster than the
@@ -1567,6 +1568,9 @@ struct ng_engine
       load += o.load;
     }
   };
+
+  // largest layout that is one allocation
+  static constexpr size_t OWN_ONE_ALLOC = 64u << 20;
 
   // Parts of less than one SM's share of the load (neurons without any
   // connection, small networks beside a large one) are joined with their
@@ -1766,6 +1770,17 @@ struct ng_engine
     const size_t p_cta = place( cta.size() * sizeof( OwnCta ) ), p_rpb = place( rpb.size() * 8 ), p_eb = place( rpb.size() * 8 ),
                  p_ebf = place( rpb.size() * 8 ), p_x = place( x_bytes ), p_rp = place( ( size_t ) rp_n * 4 ),
                  p_rpf = place( o.far ? ( size_t ) rp_n * 4 : 0 );
+    // 2-byte edge words where (delay, local target) fits 15 bits
+    o.w16 = cell == OW_COUNT && ( int64_t ) ( cfg.max_delay + 1 ) * nl < 32768 ? 1 : 0;
+    const size_t wb = cell == OW_I64 ? 8 : o.w16 ? 2 : 4, e_bytes = wb + ( cell == OW_F64 ? 8 : 0 );
+    // An allocation above 1 MB takes 0.4 ms, whatever its size: where tables and
+    // words (and weights) would both be one, the words lie beside the tables,
+    // in room for the most they can be (up to three padding edges per
+    // segment) unless that is a lot.
+    const size_t e_real = ( size_t ) own_edges_of( id );
+    const size_t e_most = ( e_real + 3 * std::min( e_real, ( size_t ) rp_n * ( o.far ? 2 : 1 ) ) ) * e_bytes + 256;
+    const bool beside = at > ( 1u << 20 ) && e_most > ( 1u << 20 ) && at + e_most <= OWN_ONE_ALLOC;
+    const size_t p_word = place( beside ? e_most : 0 );
     if ( ( rc = reserve( own_tab, at ) ) || ( !pk.p && ( rc = alloc( pk, sizeof( PkCtl ) ) ) ) )
       return rc;
     char* const tab = ( char* ) own_tab.p;
@@ -1804,12 +1819,13 @@ struct ng_engine
     const size_t edges = 4 * ( size_t ) ( quads + quads_far );
     own_edges = ( int64_t ) edges;
     own_far_edges = 4 * quads_far;
-    // 2-byte edge words where (delay, local target) fits 15 bits
-    o.w16 = cell == OW_COUNT && ( int64_t ) ( cfg.max_delay + 1 ) * nl < 32768 ? 1 : 0;
-    const size_t wb = cell == OW_I64 ? 8 : o.w16 ? 2 : 4, word_bytes = ( edges * wb + 255 ) & ~( size_t ) 255;
-    if ( ( rc = reserve( own_word, word_bytes + ( cell == OW_F64 ? edges * 8 : 0 ) ) ) )
+    const size_t word_bytes = ( edges * wb + 255 ) & ~( size_t ) 255;
+    if ( beside )
+      release( own_word );
+    else if ( ( rc = reserve( own_word, word_bytes + ( cell == OW_F64 ? edges * 8 : 0 ) ) ) )
       return rc;
-    double* const weight = ( double* ) ( ( char* ) own_word.p + word_bytes );
+    uint32_t* const word = ( uint32_t* ) ( beside ? tab + p_word : ( char* ) own_word.p );
+    double* const weight = ( double* ) ( ( char* ) word + word_bytes );
     CU( cudaMemcpyAsync( tab + p_eb, eb.data(), eb.size() * 8, cudaMemcpyHostToDevice, stream ) );
     CU( cudaMemcpyAsync( tab + p_ebf, ebf.data(), ebf.size() * 8, cudaMemcpyHostToDevice, stream ) );
     // rows of many edges per segment by one CTA each, others by a warp (the
@@ -1819,7 +1835,7 @@ struct ng_engine
     if ( !rows )
     {
       k_own_pad<<< ( unsigned ) ( 16 * sms ), 256, 0, stream >>>( o.w16, cell == OW_I64 ? 1 : 0, edges,
-        ( uint32_t ) ( md * nl + nl - 1 ), ( uint32_t* ) own_word.p );
+        ( uint32_t ) ( md * nl + nl - 1 ), word );
       if ( cell == OW_F64 )
         CU( cudaMemsetAsync( weight, 0, edges * 8, stream ) );
     }
@@ -1831,7 +1847,6 @@ struct ng_engine
     each_part( rows ? 1 : 8, [ & ]( unsigned g ) {
       const long long* const near = ( const long long* ) ( tab + p_eb );
       const long long* const far = ( const long long* ) ( tab + p_ebf );
-      uint32_t* const word = ( uint32_t* ) own_word.p;
       const uint32_t pad = ( uint32_t ) ( md * nl + nl - 1 );
       if ( rows && cell == OW_COUNT )
         k_own_fill_rows< T, OW_COUNT ><<< g, 512, OW_FILL_SMEM, stream >>>( q, o.w16, nl, pad, near, far, word, weight );
@@ -1857,8 +1872,8 @@ struct ng_engine
     o.e_base = ( const long long* ) ( tab + p_eb );
     o.rp_far = q.rp_far;
     o.e_far = ( const long long* ) ( tab + p_ebf );
-    o.word = ( const uint4* ) own_word.p;
-    o.word_w = ( const uint4* ) own_word.p;
+    o.word = ( const uint4* ) word;
+    o.word_w = ( const uint4* ) word;
     o.weight = ( const double2* ) weight;
     o.xchg = ( unsigned long long* ) own_x;
     o.nl = nl;
