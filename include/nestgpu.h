@@ -300,9 +300,10 @@ int ng_get_tuning( ng_engine* eng, ng_tuning* out );
 #define NG_FORM_OWNED 4    /* k_run_owned: many slices in one launch, each SM owning its targets */
 
 /* NG_FORM_OWNED keeps a copy of the network's edges, grouped by the SM that owns
- * their targets: 2 to 12 bytes per edge and 4 bytes per neuron and SM, held until the
- * graph changes (serving engines: until the last network is removed) or another
- * form is chosen.  It is built by ng_simulate (100 us below 1e5 edges, some 0.7 ms
+ * their targets: 2 to 12 bytes per edge (those of one source to one SM padded to a
+ * multiple of four) and 4 bytes per neuron and SM, held until the graph changes
+ * (serving engines: until the last network is removed) or another form is
+ * chosen.  It is built by ng_simulate (100 us below 1e5 edges, some 0.7 ms
  * plus 45 us per 1e6 edges, 9 ms at 4.6e8) once the slices run since the graph
  * changed, with the call's, repay it -- 15 slices below 1e5 edges, 50 to 250
  * above -- and at once where ng_set_tuning fixed update variant 5; shorter calls
